@@ -24,6 +24,7 @@ UNITS = {
     "linalg.cu": [],
     "wave.cu": [],
     "lanewave.cu": [],
+    "lanepack.cu": [],
     "api.cu": [],
     "noalloc.cu": [],
     "batch.cu": [],

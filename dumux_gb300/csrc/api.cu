@@ -595,6 +595,9 @@ void tabulate(dxg_ctx* c, const dxg_problem_desc* d)
     c->line2dMs = 0.0;
     c->laneHandoff.release();
     c->laneHandoffBytes = 0;
+    c->packPlan = LanePackPlan{};
+    c->packPlanned = false;
+    c->packMem.release();
     c->waveTuneCount = 0;
     c->dropGraphs();   // the captured chunks hold the old buffers' addresses
     DXG_CUDA(cudaMemsetAsync(c->counters.get(), 0, 8 * sizeof(unsigned), st));
@@ -761,6 +764,9 @@ void tabulateMpfa(dxg_ctx* c, const dxg_problem_desc* d)
     c->laneTuneMs = 0.0;
     c->laneHandoff.release();
     c->laneHandoffBytes = 0;
+    c->packPlan = LanePackPlan{};
+    c->packPlanned = false;
+    c->packMem.release();
     c->waveTuneCount = 0;
     c->dropGraphs();
     DXG_CUDA(cudaMemsetAsync(c->counters.get(), 0, 8 * sizeof(unsigned), st));
@@ -1126,6 +1132,71 @@ LaneWaveArgs<T> laneArgs(dxg_ctx* c, const T* A, const T* L, const T* Dinv, cons
     return w;
 }
 
+// The lane sweeps over packed records apply the preconditioner wherever their plan fits, unless
+// dxg_set_lane_ring fixed another form (one launch and no level barrier: 64x64x32 2x2 blocks
+// 0.129 ms per apply against 0.195 ms for the register form and 0.345 ms for the cluster
+// wavefront, in FP32 0.068, 0.156 and 0.207 ms; 2D 100x100 1x1 0.056 ms against 0.097 ms for the
+// one-CTA line sweeps and 0.193 ms, 10x10 0.0085 against 0.015 and 0.023 ms).
+bool usePack(const dxg_ctx* c)
+{
+    return c->packPlan.ok && c->laneRingMode == 0 && c->linearSolver == DXG_LINEAR_SOLVER_ILU_BICGSTAB &&
+           (c->iluKernel == DXG_ILU_LANES || c->iluKernel == DXG_ILU_AUTO);
+}
+
+template <class T>
+LanePackArgs<T> packArgs(dxg_ctx* c, const T* A, const T* L, const T* Dinv, const T* rhs, T* v)
+{
+    const LanePackPlan& p = c->packPlan;
+    LanePackArgs<T> a{};
+    a.nx = c->pcHost.nx;
+    a.ny = c->pcHost.ny;
+    a.nz = c->dim == 3 ? c->pcHost.nz : 1;
+    a.N = c->N;
+    a.nyb = p.nyb;
+    a.warps = p.warps;
+    a.steps = p.steps;
+    a.stages = p.stages;
+    a.ctas = p.ctas;
+    a.clusterSize = p.clusterSize;
+    a.Lf = L;
+    a.A = A;
+    a.Dinv = Dinv;
+    a.pack[0] = c->packMem.get();
+    a.pack[1] = a.pack[0] + lanePackBytes(p, 1, sizeof(T));
+    a.handoff = reinterpret_cast<T*>(a.pack[1] + lanePackBytes(p, -1, sizeof(T)));
+    a.rhs = rhs;
+    a.v = v;
+    a.err = c->singular.get() + 1;
+    a.ks = c->ks.get();
+    a.waitNs = c->waitNs ? c->waitNs : 500000000ull;
+    return a;
+}
+
+// Before a factorisation: plans the packed sweeps and makes their buffers on first use.  Where
+// the records do not fit into device memory the context goes on without them.
+template <class T>
+void preparePack(dxg_ctx* c)
+{
+    if (!c->packPlanned) {
+        c->packPlanned = true;
+        c->packPlan = makeLanePackPlan<T>(c->dim, (int)c->pcHost.nx, (int)c->pcHost.ny, c->dim == 3 ? (int)c->pcHost.nz : 1,
+                                          c->b);
+    }
+    if (!usePack(c) || c->packMem.get()) return;
+    const LanePackPlan& p = c->packPlan;
+    const size_t records = lanePackBytes(p, 1, sizeof(T)) + lanePackBytes(p, -1, sizeof(T));
+    const size_t handoff = laneHandoffBytes(p, sizeof(T));
+    try {
+        c->packMem.alloc(records + handoff);
+    } catch (const Error& e) {
+        if (e.status != DXG_ERR_OOM) throw;
+        cudaGetLastError();
+        c->packPlan.ok = false;
+        return;
+    }
+    DXG_CUDA(cudaMemsetAsync(c->packMem.get() + records, 0xff, handoff, c->stream));
+}
+
 template <class T>
 RbArgs<T> rbArgs(dxg_ctx* c, const T* A, T* Dinv)
 {
@@ -1301,6 +1372,10 @@ int64_t iluApply(dxg_ctx* c, const IluArgs<T, T>& ia, const T* A, T* L, T* Dinv,
 {
     TimedScope ts(c, DXG_KC_ILU_SWEEP, c->bytesSweep * sizeof(T) / 8.0);
     if (c->iluKernel == DXG_ILU_REDBLACK) return launchRbApply<T>(rbArgs<T>(c, A, Dinv), c->b, c->dim, d, v, c->stream);
+    if (usePack(c)) {
+        launchLanePackApply<T>(c->packPlan, packArgs<T>(c, A, L, Dinv, d, v), c->stream);
+        return 1;
+    }
     if (useLine2d(c)) {
         const LaneWaveArgs<T> la = line2dArgs<T>(c, A, L, Dinv, d, v);
         launchTpfaLine2d<T>(la, la, c->b, c->stream);
@@ -1379,6 +1454,13 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
         } else {
             c->launches += launchIluFactor<PT>(ia, c->levels, c->b, c->dim, st);
         }
+        if (!c->mpfa) {
+            preparePack<PT>(c);
+            if (usePack(c)) {
+                launchLanePack<PT>(c->packPlan, packArgs<PT>(c, PA, PL, PD, nullptr, nullptr), st);
+                c->launches += 1;
+            }
+        }
     }
     double *x = c->kx.get(), *r = c->kr.get(), *rt = c->krt.get(), *p = c->kp.get(), *v = c->kv.get(),
            *t = c->kt.get(), *y = c->ky.get();
@@ -1411,7 +1493,7 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
     sv.ks = c->ks.get();
     sv.scratch = c->scratch();
     const bool amg = c->linearSolver == DXG_LINEAR_SOLVER_AMG_BICGSTAB;
-    if (refactor && !amg && useWave(c) && !c->waveTuned) tuneWavePlan<PT>(c, PA, PL, PD, pIn, yOut);
+    if (refactor && !amg && useWave(c) && !c->waveTuned && !usePack(c)) tuneWavePlan<PT>(c, PA, PL, PD, pIn, yOut);
     std::vector<AmgLevel<PT>> amgP, amgR;
     if (amg) {
         amgP = amgLevels<PT>(c, PA, PD, pIn, yOut);
@@ -1475,7 +1557,7 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
     const int chunk = graphs ? 8 : 4;
     dxg_ctx::ChunkGraph& G = c->chunkGraph[mixed ? 1 : 0];
     if (graphs) {
-        const int key[4] = {c->iluKernel + 16 * c->linearSolver, useLane(c) ? -1 : useWave(c) ? c->wavePlan.ctas : 0,
+        const int key[4] = {c->iluKernel + 16 * c->linearSolver, usePack(c) ? -2 : useLane(c) ? -1 : useWave(c) ? c->wavePlan.ctas : 0,
                             useWave(c) ? c->wavePlan.threads : 0, chunk};
         if (G.exec && !std::equal(key, key + 4, G.key)) {
             cudaGraphExecDestroy(G.exec);
@@ -1521,6 +1603,10 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
         // a sweep that gave up may leave hand-off entries written: start the next from scratch
         if (c->laneHandoffBytes)
             DXG_CUDA(cudaMemsetAsync(c->laneHandoff.get(), 0xff, c->laneHandoffBytes, st));
+        if (c->packMem.get()) {
+            const size_t ts = sizeof(PT), handoff = laneHandoffBytes(c->packPlan, ts);
+            DXG_CUDA(cudaMemsetAsync(c->packMem.get() + c->packMem.bytes() - handoff, 0xff, handoff, st));
+        }
         DXG_CUDA(cudaMemsetAsync(c->singular.get() + 1, 0, sizeof(int), st));
         DXG_CUDA(cudaStreamSynchronize(st));
         throw Error(DXG_ERR_TIMEOUT, "ILU(0) wavefront wait timed out");
@@ -2124,6 +2210,11 @@ int dxg_describe(const dxg_ctx* c, char* buf, int64_t len)
                                                                (int)c->pcHost.nz).size() + 1) +
               " levels of 2x2(x2) aggregation, damped block-Jacobi smoothing";
     else if (c->iluKernel == DXG_ILU_REDBLACK) out = "ILU(0): red-black ordering, two parallel passes per sweep";
+    else if (usePack(c)) {
+        out = "ILU(0): lane wavefront (packed records), " + std::to_string(c->packPlan.ctas) + " CTAs of " +
+              std::to_string(c->packPlan.warps) + " warps in clusters of " + std::to_string(c->packPlan.clusterSize) +
+              ", both sweeps in one launch";
+    }
     else if (useLine2d(c)) {
         out = "ILU(0): line sweeps in one CTA (one thread per grid line, levels x+y)";
         if (c->line2dMs > 0) {

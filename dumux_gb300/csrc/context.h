@@ -118,6 +118,11 @@ struct dxg_ctx {
     bool line2dOk = false;         // the one-CTA line sweeps of 2D TPFA systems fit
     bool line2d = false;           // ... and the timing at the first factorisation chose them
     double line2dMs = 0.0;
+    // lane sweeps over packed records (lanepack.cu): the default natural-order apply wherever their
+    // plan fits; planned at the first factorisation that uses them
+    dxg::LanePackPlan packPlan;
+    bool packPlanned = false;
+    dxg::DevBuf<unsigned char> packMem;   // records of both sweeps, then the hand-off buffer
     dxg::DevBuf<unsigned char> laneHandoff;
     size_t laneHandoffBytes = 0;
     // limit of every bounded wait of the sweeps (0: the kernels' default, 0.5 s)

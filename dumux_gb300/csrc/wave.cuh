@@ -58,6 +58,41 @@ template <class T>
 LanePlan makeLanePlan(int dim, int nx, int ny, int nz, int b);
 template <class T>
 void launchLaneWaveApply(const LanePlan& p, const LaneWaveArgs<T>& fwd, const LaneWaveArgs<T>& bwd, cudaStream_t st);
+// Sweeps of lanepack.cu (2D and 3D, 1x1 and 2x2 blocks): one lane per grid line and block row,
+// tiles of one z-plane spread over thread-block clusters, the factor packed per warp and step.
+template <class T>
+struct LanePackArgs {
+    int nx, ny, nz;
+    int64_t N;
+    int nyb, warps, steps;    // CTAs per plane, warps per CTA, padded steps per warp
+    int stages;               // depth of the record ring
+    int ctas;                 // working CTAs (nz * nyb); the grid is padded to whole clusters
+    int clusterSize;
+    const T* Lf;              // pack: lower factor, matrix (upper slots), inverted pivots
+    const T* A;
+    const T* Dinv;
+    unsigned char* pack[2];   // packed records of the forward / backward sweep
+    const T* rhs;             // forward input
+    T* v;                     // forward output, backward in/out
+    int* err;                 // DXG_ERR_TIMEOUT on an expired wait
+    const KrylovState* ks;    // sweeps are skipped once the solve has stopped
+    T* handoff;               // [2][ctas][warps][steps][32 rows], all bits set between launches
+    unsigned long long waitNs;
+};
+struct LanePackPlan {
+    bool ok = false;
+    int dim = 0, b = 0, nyb = 0, warps = 0, steps = 0, ctas = 0, clusterSize = 0, grid = 0;
+    int rows = 0, stages = 0;   // rows per lane, depth of the record ring
+};
+// The plan of a grid (ok: shared memory holds the histories and every cluster is resident).
+template <class T>
+LanePackPlan makeLanePackPlan(int dim, int nx, int ny, int nz, int b);
+size_t lanePackBytes(const LanePackPlan& p, int dir, size_t tsize);
+size_t laneHandoffBytes(const LanePackPlan& p, size_t tsize);
+template <class T>
+void launchLanePack(const LanePackPlan& p, const LanePackArgs<T>& a, cudaStream_t st);
+template <class T>
+void launchLanePackApply(const LanePackPlan& p, const LanePackArgs<T>& a, cudaStream_t st);
 // One-CTA line sweeps of 2D cc-TPFA systems (linesweep.cu): one thread per grid line, both block
 // rows, for grids of up to 512 lines; uses nx, ny, N, Lf, A, Dinv, rhs, v and ks of the args.
 bool tpfaLine2dFits(int dim, int nx, int ny, int b);

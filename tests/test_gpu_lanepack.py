@@ -1,0 +1,67 @@
+"""The lane sweeps over packed records against the cluster wavefront (the same arithmetic, so the
+same bits) at the edges of their tiles, warps and clusters, and their bounded waits."""
+import numpy as np
+import pytest
+
+from dumux_gb300 import Context, problems
+
+pytestmark = pytest.mark.gpu
+
+
+def _solve(desc, u, prev, kind, precision, dt):
+    ctx = Context(desc, precision=precision)
+    ctx.set_ilu_kernel(kind)
+    ctx.set_solution(u)
+    if dt:
+        ctx.set_prev_solution(prev)
+        ctx.set_time_step(dt)
+    ctx.assemble_jacobian_and_residual()
+    res = ctx.linear_solve(1e-10 if precision == "fp64" else 1e-4, 400)
+    return res["iterations"], ctx.update(), ctx.describe()
+
+
+# lines per warp: 16 (2x2 FP64) or 32; up to three warps per CTA; 16 CTAs per cluster
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("eqs,dims", [
+    (1, (1, 1)), (1, (5, 32)), (1, (40, 33)), (1, (7, 97)), (1, (300, 3)),
+    (1, (3, 5, 17)), (1, (9, 33, 5)), (1, (6, 70, 18)), (1, (20, 8, 33)),
+    (2, (4, 16)), (2, (30, 17)), (2, (6, 49, 3)), (2, (8, 15, 16)), (2, (5, 33, 17)), (2, (12, 97, 6)), (2, (3, 2, 40)),
+])
+def test_packed_lane_sweeps_equal_cluster_wavefront(eqs, dims, precision):
+    if eqs == 1:
+        desc, u = problems.darcy_1p(cells=dims, seed=4)
+        prev, dt = u, 0.0
+    else:
+        desc, prev = problems.dnapl_2p(cells=dims, extent=(6.0, 4.0, 1.0)[:len(dims)], seed=4)
+        u = prev.reshape(-1, 2).copy()
+        u[:, 1] = np.random.default_rng(3).uniform(0.0, 0.3, len(u))
+        u, dt = u.reshape(-1), 250.0
+    n0, x0, _ = _solve(desc, u, prev, "wavefront", precision, dt)
+    n1, x1, how = _solve(desc, u, prev, "auto", precision, dt)
+    assert "packed records" in how
+    assert n1 == n0
+    assert np.array_equal(x1, x0)
+
+
+def test_packed_lane_sweeps_wait_limit_expires_and_the_context_recovers():
+    """A wait limit far below the time the last of 40 planes waits for its first value: the sweeps
+    give up, the solve reports DXG_ERR_TIMEOUT, and with the limit restored the context solves to
+    the same bits (the hand-off buffer between clusters is reset)."""
+    desc, u0 = problems.dnapl_2p(cells=(16, 16, 40), seed=8)
+    u = u0.reshape(-1, 2).copy()
+    u[:, 1] = np.random.default_rng(5).uniform(0.0, 0.4, len(u))
+    ctx = Context(desc)
+    ctx.set_solution(u.reshape(-1))
+    ctx.set_prev_solution(u0)
+    ctx.set_time_step(250.0)
+    ctx.assemble_jacobian_and_residual()
+    first = ctx.linear_solve(1e-10, 500)
+    assert first["converged"] and "packed records" in ctx.describe()
+    x0 = ctx.update()
+    ctx.set_wait_limit(1e-6)
+    with pytest.raises(Exception, match="timed out"):
+        ctx.linear_solve(1e-10, 500)
+    ctx.set_wait_limit(0.5)
+    again = ctx.linear_solve(1e-10, 500)
+    assert again["converged"] and again["iterations"] == first["iterations"]
+    assert np.array_equal(ctx.update(), x0)
