@@ -284,6 +284,7 @@ __device__ __forceinline__ void coarseRow(const AmgLevel<T>& L, int n, int i)
 template <int B, class T>
 __global__ void amgFirstKernel(AmgLevel<T> L, T* out, T omega, const KrylovState* ks)
 {
+    chainWait();
     if (stopped<T>(ks)) return;
     AMG_LOOP(L) firstCell<B, T>(L, i, out, omega);
 }
@@ -292,6 +293,7 @@ template <int B, int DIM, class T>
 __global__ void amgJacobiKernel(AmgLevel<T> L, const T* xin, const T* xc, int cnx, int cny, T* out, T omega,
                                 const KrylovState* ks)
 {
+    chainWait();
     if (stopped<T>(ks)) return;
     AMG_LOOP(L) jacobiCell<B, DIM, T>(L, i, xin, xc, cnx, cny, out, omega);
 }
@@ -299,6 +301,7 @@ __global__ void amgJacobiKernel(AmgLevel<T> L, const T* xin, const T* xc, int cn
 template <int B, int DIM, class T>
 __global__ void amgResidualKernel(AmgLevel<T> L, const T* xin, const KrylovState* ks)
 {
+    chainWait();
     if (stopped<T>(ks)) return;
     AMG_LOOP(L) residualCell<B, DIM, T>(L, i, xin);
 }
@@ -306,6 +309,7 @@ __global__ void amgResidualKernel(AmgLevel<T> L, const T* xin, const KrylovState
 template <int B, int DIM, class T>
 __global__ void amgRestrictKernel(AmgLevel<T> F, AmgLevel<T> C, const KrylovState* ks)
 {
+    chainWait();
     if (stopped<T>(ks)) return;
     AMG_LOOP(C) restrictCell<B, DIM, T>(F, C, i);
 }
@@ -326,6 +330,7 @@ struct AmgCycle {
 template <int B, int DIM, class T>
 __global__ void __launch_bounds__(kAmgClusterThreads) amgClusterCycle(AmgCycle<T> cy, const KrylovState* ks)
 {
+    chainWait();
     if (stopped<T>(ks)) return;   // uniform: the status does not change during the launch
     cg::cluster_group cl = cg::this_cluster();
     const int64_t gid = (int64_t)cl.block_rank() * blockDim.x + threadIdx.x;
@@ -472,6 +477,7 @@ __global__ void amgCoarseInvertKernel(AmgLevel<T> L, int* singular)
 template <class T>
 __global__ void amgCoarseSolveKernel(AmgLevel<T> L, int n, const KrylovState* ks)
 {
+    chainWait();
     if (stopped<T>(ks)) return;
     for (int i = threadIdx.x; i < n; i += blockDim.x) coarseRow<T>(L, n, i);
 }
@@ -536,18 +542,20 @@ int64_t vcycle(const std::vector<AmgLevel<T>>& Ls, size_t l, const KrylovState* 
         cfg.gridDim = dim3(kAmgClusterCtas);
         cfg.blockDim = dim3(kAmgClusterThreads);
         cfg.stream = st;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = kAmgClusterCtas;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 2;
         DXG_CUDA(cudaLaunchKernelEx(&cfg, kern, cy, ks));
         return 1;
     }
     if (l + 1 == Ls.size()) {
-        amgCoarseSolveKernel<T><<<1, kAmgThreads, 0, st>>>(L, (int)L.N * B, ks);   // exact solve
+        launchChained(amgCoarseSolveKernel<T>, dim3(1), kAmgThreads, st, L, (int)L.N * B, ks);   // exact solve
         return 1;
     }
     const AmgLevel<T>& C = Ls[l + 1];
@@ -556,22 +564,22 @@ int64_t vcycle(const std::vector<AmgLevel<T>>& Ls, size_t l, const KrylovState* 
     // 2*sweeps writes alternate between tmp and x, the last one into x
     T* buf[2] = {L.tmp, L.x};
     int w = 0;
-    amgFirstKernel<B, T><<<g, kAmgThreads, 0, st>>>(L, buf[w & 1], omega, ks);
+    launchChained(amgFirstKernel<B, T>, dim3(g), kAmgThreads, st, L, buf[w & 1], omega, ks);
     ++n;
     for (int k = 1; k < L.sweeps; ++k, ++w, ++n)
-        amgJacobiKernel<B, DIM, T><<<g, kAmgThreads, 0, st>>>(L, buf[w & 1], nullptr, 0, 0, buf[(w + 1) & 1], omega,
+        launchChained(amgJacobiKernel<B, DIM, T>, dim3(g), kAmgThreads, st, L, buf[w & 1], nullptr, 0, 0, buf[(w + 1) & 1], omega,
                                                               ks);
     const T* pre = buf[w & 1];
-    amgResidualKernel<B, DIM, T><<<g, kAmgThreads, 0, st>>>(L, pre, ks);
-    amgRestrictKernel<B, DIM, T><<<gridFor(C.N), kAmgThreads, 0, st>>>(L, C, ks);
+    launchChained(amgResidualKernel<B, DIM, T>, dim3(g), kAmgThreads, st, L, pre, ks);
+    launchChained(amgRestrictKernel<B, DIM, T>, dim3(gridFor(C.N)), kAmgThreads, st, L, C, ks);
     n += 2;
     n += vcycle<T, B, DIM>(Ls, l + 1, ks, st);
     // prolongation fused into the first post-sweep
-    amgJacobiKernel<B, DIM, T><<<g, kAmgThreads, 0, st>>>(L, pre, C.x, C.nx, C.ny, buf[(w + 1) & 1], omega, ks);
+    launchChained(amgJacobiKernel<B, DIM, T>, dim3(g), kAmgThreads, st, L, pre, C.x, C.nx, C.ny, buf[(w + 1) & 1], omega, ks);
     ++w;
     ++n;
     for (int k = 1; k < L.sweeps; ++k, ++w, ++n)
-        amgJacobiKernel<B, DIM, T><<<g, kAmgThreads, 0, st>>>(L, buf[w & 1], nullptr, 0, 0, buf[(w + 1) & 1], omega,
+        launchChained(amgJacobiKernel<B, DIM, T>, dim3(g), kAmgThreads, st, L, buf[w & 1], nullptr, 0, 0, buf[(w + 1) & 1], omega,
                                                               ks);
     return n;
 }

@@ -38,25 +38,37 @@ __device__ __forceinline__ double warpMax(double v)
     return v;
 }
 
-// Block-wide sum of NV values per thread; result valid in thread 0.
+// Block-wide sum of NV values per thread (256 threads); result valid in thread 0.  The sums are
+// those of a butterfly over each warp and then over the warps' sums, (((v0 + v16) + (v8 + v24)) +
+// ...), but of every butterfly only the additions that reach lane 0 are done, on the values of
+// all warps side by side: an FP64 warp instruction costs the same 64 cycles for one lane as for
+// 32, and the butterflies of a one-row-per-thread kernel took a quarter of its FP64 instructions
+// (90 per block and pair of sums; here 27).
 template <int NV>
 __device__ __forceinline__ void blockSum(double (&v)[NV])
 {
-    __shared__ double sh[NV][32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    static_assert(kReduceThreads == 256 && NV * 64 <= kReduceThreads, "");
+    __shared__ double sh[NV][kReduceThreads];
+    __shared__ double warps[NV][8];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = warpSum(v[k]);
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) sh[k][wid] = v[k];
+    for (int k = 0; k < NV; ++k) sh[k][threadIdx.x] = v[k];
     __syncthreads();
-    if (wid == 0) {
-        const int nw = blockDim.x >> 5;
+    if (threadIdx.x < NV * 64) {
+        const int k = threadIdx.x >> 6, w = (threadIdx.x >> 3) & 7, m = threadIdx.x & 7;
+        const double* q = &sh[k][w * 32 + m];
+        double t = (q[0] + q[16]) + (q[8] + q[24]);
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double t = lane < nw ? sh[k][lane] : 0.0;
-            v[k] = warpSum(t);
-        }
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (m == 0) warps[k][w] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int k = (threadIdx.x >> 3) < NV ? threadIdx.x >> 3 : 0;
+        double t = warps[k][threadIdx.x & 7];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+#pragma unroll
+        for (int e = 0; e < NV; ++e) v[e] = __shfl_sync(0xffffffffu, t, 8 * e);
     }
 }
 
@@ -111,16 +123,29 @@ __device__ __forceinline__ bool gridSum(double (&v)[NV], double* partials, unsig
     __syncthreads();
     if (!amLast) return false;
     __threadfence();
-    // the last block combines the partials in block order
-    if (threadIdx.x < 32) {
+    // The last block combines the partials in block order: lane l sums those of blocks l, l + 32,
+    // ..., then the warp sums the lanes.  All partials are fetched at once (one after another, each
+    // addition would wait for a trip to L2: 16 of them at 512 blocks took longer than the rest of
+    // the kernel), sum k by warp k.
+    __shared__ double all[NV][kMaxReduceBlocks];
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double s = 0.0;
-            for (unsigned bI = threadIdx.x; bI < nblk; bI += 32)
-                s += ((volatile double*)partials)[k * kMaxReduceBlocks + bI];
-            v[k] = warpSum(s);
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+        for (int e = 0; e < kMaxReduceBlocks / kReduceThreads; ++e) {
+            const unsigned bI = threadIdx.x + e * kReduceThreads;
+            if (bI < nblk) all[k][bI] = __ldcg(partials + k * kMaxReduceBlocks + bI);
         }
+    __syncthreads();
+    const unsigned wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (wid < NV) {
+        double s = 0.0;
+        for (unsigned bI = lane; bI < nblk; bI += 32) s += all[wid][bI];
+        s = warpSum(s);
+        if (lane == 0) all[wid][0] = s;
     }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = all[k][0];
     if (threadIdx.x == 0) *counter = 0u;
     return threadIdx.x == 0;
 }
@@ -199,12 +224,34 @@ __device__ __forceinline__ bool slotValid(unsigned mask, int dim, int s)
     return (mask >> f) & 1u;
 }
 
+// The value of a float as a double, from the bits (the exponent rebiased, the mantissa shifted;
+// subnormals normalised): the conversion instruction runs at the FP64 rate, and a row of the
+// mixed-precision SpMV would need one for every second product.  No path may use it: the
+// compiler would issue it speculatively.
+__device__ __forceinline__ double widen(float f)
+{
+    const uint32_t u = __float_as_uint(f), sign = u & 0x80000000u;
+    uint32_t mag = u & 0x7fffffffu, bias = mag ? 0x38000000u : 0u;   // 1023 - 127
+    if (mag - 0x00800000u >= 0x7f000000u && mag != 0u) {
+        if (mag >= 0x7f800000u) {
+            bias = 0x70000000u;                                      // infinities, NaNs: 2047 - 255
+        } else {
+            const int shift = __clz((int)mag) - 8;                   // subnormals
+            mag = (mag << shift) & 0x007fffffu;
+            bias = (uint32_t)(897 - shift) << 20;
+        }
+    }
+    return __hiloint2double((int)(((mag >> 3) + bias) | sign), (int)(mag << 29));
+}
+__device__ __forceinline__ double widen(double f) { return f; }
+
 // ---------------------------------------------------------------- SpMV
 // y = A x; MODE 0: plain; MODE 1: also dot(w, y) -> h, alpha; MODE 2: dots (y,w),(y,y) -> omega
 template <int B, int DIM, class MT, class VT, class XT, int MODE>
-__global__ void __launch_bounds__(kReduceThreads) spmvKernel(SpmvArgs<MT, VT, XT> a0,
+__global__ void __launch_bounds__(kReduceThreads, 4) spmvKernel(SpmvArgs<MT, VT, XT> a0,
                                                               const SpmvArgs<MT, VT, XT>* batch, const uint2* map)
 {
+    chainWait();
     // accumulation: FP32 when both operands are FP32, else the output type
     using AT = typename std::conditional<sizeof(MT) == 4 && sizeof(XT) == 4, float, VT>::type;
     unsigned lb;
@@ -232,7 +279,10 @@ __global__ void __launch_bounds__(kReduceThreads) spmvKernel(SpmvArgs<MT, VT, XT
             ldgVec<B>(a.x + (i + (valid ? a.off[s] : 0)) * B, xs);
             AT xj[B];
 #pragma unroll
-            for (int e = 0; e < B; ++e) xj[e] = valid ? (AT)xs[e] : (AT)0;
+            for (int e = 0; e < B; ++e) {
+                if constexpr (sizeof(AT) == 8) xj[e] = valid ? widen(xs[e]) : 0.0;
+                else xj[e] = valid ? (AT)xs[e] : (AT)0;
+            }
 #pragma unroll
             for (int e = 0; e < BB; ++e) blk[e] = valid ? blk[e] : (MT)0;
             blkMv<B>(blk, xj, sum);
@@ -427,6 +477,7 @@ __global__ void rbFactorBlack(RbArgs<T> a0, const RbArgs<T>* batch, const uint2*
 template <int B, int DIM, class T>
 __global__ void rbApplyBlack(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* map)
 {
+    chainWait();
     unsigned lb;
     const RbArgs<T> a = problemOf(a0, batch, map, lb);
     if (a.ks && a.ks->status != KS_RUNNING) return;
@@ -478,6 +529,7 @@ __global__ void rbApplyBlack(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* 
 template <int B, int DIM, class T>
 __global__ void rbApplyRed(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* map)
 {
+    chainWait();
     unsigned lb;
     const RbArgs<T> a = problemOf(a0, batch, map, lb);
     if (a.ks && a.ks->status != KS_RUNNING) return;
@@ -633,6 +685,7 @@ __global__ void __launch_bounds__(kReduceThreads) bicgInit(BicgArgs<VT> a0, cons
 template <class VT>
 __global__ void bicgUpdateP(BicgArgs<VT> a0, const BicgArgs<VT>* batch, const uint2* map)
 {
+    chainWait();
     DXG_PROBLEM_BLOCKS(BicgArgs<VT>, M)
     const KrylovState& ks = *a.ks;
     if (ks.status != KS_RUNNING) return;
@@ -657,6 +710,7 @@ __global__ void bicgUpdateP(BicgArgs<VT> a0, const BicgArgs<VT>* batch, const ui
 template <class VT, int STAGE>
 __global__ void __launch_bounds__(kReduceThreads) bicgAxpyNorm(BicgArgs<VT> a0, const BicgArgs<VT>* batch, const uint2* map)
 {
+    chainWait();
     DXG_PROBLEM_BLOCKS(BicgArgs<VT>, M)
     const KrylovState& ksr = *a.ks;
     if (ksr.status != KS_RUNNING) return;
@@ -719,12 +773,19 @@ __global__ void __launch_bounds__(kReduceThreads) newtonUpdateKernel(NewtonUpdAr
         amLast = atomicAdd(counter, 1u) == nblk - 1;
     }
     __syncthreads();
-    if (amLast && threadIdx.x == 0) {
+    if (amLast) {
+        // the maximum of the blocks' maxima, fetched by all threads at once
         __threadfence();
         double g = 0.0;
-        for (unsigned bI = 0; bI < nblk; ++bI) g = fmax(g, ((volatile double*)partials)[bI]);
-        *a.shiftOut = g;
-        *counter = 0u;
+        for (unsigned bI = threadIdx.x; bI < nblk; bI += blockDim.x) g = fmax(g, __ldcg(partials + bI));
+        g = warpMax(g);
+        if (lane == 0) sh[wid] = g;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < (int)(blockDim.x >> 5); ++k) g = fmax(g, sh[k]);
+            *a.shiftOut = g;
+            *counter = 0u;
+        }
     }
 }
 
@@ -835,9 +896,9 @@ template <int B, int DIM, class MT, class VT, class XT>
 static void spmvT(const SpmvArgs<MT, VT, XT>& a, const SpmvArgs<MT, VT, XT>* batch, const uint2* map, dim3 g,
                   int mode, cudaStream_t st)
 {
-    if (mode == 0) spmvKernel<B, DIM, MT, VT, XT, 0><<<g, kReduceThreads, 0, st>>>(a, batch, map);
-    else if (mode == 1) spmvKernel<B, DIM, MT, VT, XT, 1><<<g, kReduceThreads, 0, st>>>(a, batch, map);
-    else spmvKernel<B, DIM, MT, VT, XT, 2><<<g, kReduceThreads, 0, st>>>(a, batch, map);
+    if (mode == 0) launchChained(spmvKernel<B, DIM, MT, VT, XT, 0>, dim3(g), kReduceThreads, st, a, batch, map);
+    else if (mode == 1) launchChained(spmvKernel<B, DIM, MT, VT, XT, 1>, dim3(g), kReduceThreads, st, a, batch, map);
+    else launchChained(spmvKernel<B, DIM, MT, VT, XT, 2>, dim3(g), kReduceThreads, st, a, batch, map);
 }
 template <class MT, class VT, class XT>
 static void spmvDispatch(const SpmvArgs<MT, VT, XT>& a, const SpmvArgs<MT, VT, XT>* batch, const uint2* map, dim3 g,
@@ -919,8 +980,8 @@ static void rbFactorPasses(const RbArgs<T>& a, const RbArgs<T>* batch, const uin
 template <class T, int B, int DIM>
 static void rbApplyPasses(const RbArgs<T>& a, const RbArgs<T>* batch, const uint2* map, unsigned g, cudaStream_t st)
 {
-    rbApplyBlack<B, DIM, T><<<g, kReduceThreads, 0, st>>>(a, batch, map);
-    rbApplyRed<B, DIM, T><<<g, kReduceThreads, 0, st>>>(a, batch, map);
+    launchChained(rbApplyBlack<B, DIM, T>, dim3(g), kReduceThreads, st, a, batch, map);
+    launchChained(rbApplyRed<B, DIM, T>, dim3(g), kReduceThreads, st, a, batch, map);
 }
 template <class T>
 static void rbDispatch(bool factor, const RbArgs<T>& a, const RbArgs<T>* batch, const uint2* map, unsigned g, int b,
@@ -975,13 +1036,13 @@ void launchBicgInit(const BicgArgs<VT>& a, const double* rhs, cudaStream_t st)
 template <class VT>
 void launchBicgUpdateP(const BicgArgs<VT>& a, cudaStream_t st)
 {
-    bicgUpdateP<VT><<<reduceBlocks(a.M), kReduceThreads, 0, st>>>(a, nullptr, nullptr);
+    launchChained(bicgUpdateP<VT>, dim3(reduceBlocks(a.M)), kReduceThreads, st, a, nullptr, nullptr);
 }
 template <class VT>
 void launchBicgAxpyNorm(const BicgArgs<VT>& a, int stage, cudaStream_t st)
 {
-    if (stage == 0) bicgAxpyNorm<VT, 0><<<reduceBlocks(a.M), kReduceThreads, 0, st>>>(a, nullptr, nullptr);
-    else bicgAxpyNorm<VT, 1><<<reduceBlocks(a.M), kReduceThreads, 0, st>>>(a, nullptr, nullptr);
+    if (stage == 0) launchChained(bicgAxpyNorm<VT, 0>, dim3(reduceBlocks(a.M)), kReduceThreads, st, a, nullptr, nullptr);
+    else launchChained(bicgAxpyNorm<VT, 1>, dim3(reduceBlocks(a.M)), kReduceThreads, st, a, nullptr, nullptr);
 }
 template <class VT>
 void launchBicgInitBatch(const BicgArgs<VT>* batch, const BlockMap& m, cudaStream_t st)
@@ -992,13 +1053,13 @@ void launchBicgInitBatch(const BicgArgs<VT>* batch, const BlockMap& m, cudaStrea
 template <class VT>
 void launchBicgUpdatePBatch(const BicgArgs<VT>* batch, const BlockMap& m, cudaStream_t st)
 {
-    bicgUpdateP<VT><<<m.blocks, kReduceThreads, 0, st>>>(BicgArgs<VT>{}, batch, m.map);
+    launchChained(bicgUpdateP<VT>, dim3(m.blocks), kReduceThreads, st, BicgArgs<VT>{}, batch, m.map);
 }
 template <class VT>
 void launchBicgAxpyNormBatch(const BicgArgs<VT>* batch, const BlockMap& m, int stage, cudaStream_t st)
 {
-    if (stage == 0) bicgAxpyNorm<VT, 0><<<m.blocks, kReduceThreads, 0, st>>>(BicgArgs<VT>{}, batch, m.map);
-    else bicgAxpyNorm<VT, 1><<<m.blocks, kReduceThreads, 0, st>>>(BicgArgs<VT>{}, batch, m.map);
+    if (stage == 0) launchChained(bicgAxpyNorm<VT, 0>, dim3(m.blocks), kReduceThreads, st, BicgArgs<VT>{}, batch, m.map);
+    else launchChained(bicgAxpyNorm<VT, 1>, dim3(m.blocks), kReduceThreads, st, BicgArgs<VT>{}, batch, m.map);
 }
 template <class VT>
 void launchCopyToDouble(const VT* x, double* y, int64_t M, cudaStream_t st)
@@ -1136,6 +1197,7 @@ template <int S, int MODE>
 __global__ void __launch_bounds__(kReduceThreads) stencilSpmvKernel(StencilArgs a, const double* __restrict__ x,
                                                                      double* __restrict__ y, const double* __restrict__ w)
 {
+    chainWait();
     const unsigned nblk = cellBlocksFor(a.N);
     const unsigned lb = blockIdx.x;
     if (a.ks && a.ks->status != KS_RUNNING) return;
@@ -1367,6 +1429,7 @@ template <int S, int MODE>
 __global__ void __launch_bounds__(kReduceThreads) stencilSpmv2Kernel(StencilArgs a, const double* __restrict__ x,
                                                                       double* __restrict__ y, const double* __restrict__ w)
 {
+    chainWait();
     const unsigned nblk = cellBlocksFor(a.N);
     const unsigned lb = blockIdx.x;
     if (a.ks && a.ks->status != KS_RUNNING) return;
@@ -1519,25 +1582,25 @@ void launchStencilSpmv(const StencilArgs& a, const double* x, double* y, const d
     const dim3 g((unsigned)cellBlocksFor(a.N));
     if (a.b == 2) {
         if (a.S == 9) {
-            if (mode == 0) stencilSpmv2Kernel<9, 0><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
-            else if (mode == 1) stencilSpmv2Kernel<9, 1><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
-            else stencilSpmv2Kernel<9, 2><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
+            if (mode == 0) launchChained(stencilSpmv2Kernel<9, 0>, dim3(g), kReduceThreads, st, a, x, y, w);
+            else if (mode == 1) launchChained(stencilSpmv2Kernel<9, 1>, dim3(g), kReduceThreads, st, a, x, y, w);
+            else launchChained(stencilSpmv2Kernel<9, 2>, dim3(g), kReduceThreads, st, a, x, y, w);
         } else {
-            if (mode == 0) stencilSpmv2Kernel<27, 0><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
-            else if (mode == 1) stencilSpmv2Kernel<27, 1><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
-            else stencilSpmv2Kernel<27, 2><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
+            if (mode == 0) launchChained(stencilSpmv2Kernel<27, 0>, dim3(g), kReduceThreads, st, a, x, y, w);
+            else if (mode == 1) launchChained(stencilSpmv2Kernel<27, 1>, dim3(g), kReduceThreads, st, a, x, y, w);
+            else launchChained(stencilSpmv2Kernel<27, 2>, dim3(g), kReduceThreads, st, a, x, y, w);
         }
         DXG_CUDA(cudaGetLastError());
         return;
     }
     if (a.S == 9) {
-        if (mode == 0) stencilSpmvKernel<9, 0><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
-        else if (mode == 1) stencilSpmvKernel<9, 1><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
-        else stencilSpmvKernel<9, 2><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
+        if (mode == 0) launchChained(stencilSpmvKernel<9, 0>, dim3(g), kReduceThreads, st, a, x, y, w);
+        else if (mode == 1) launchChained(stencilSpmvKernel<9, 1>, dim3(g), kReduceThreads, st, a, x, y, w);
+        else launchChained(stencilSpmvKernel<9, 2>, dim3(g), kReduceThreads, st, a, x, y, w);
     } else {
-        if (mode == 0) stencilSpmvKernel<27, 0><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
-        else if (mode == 1) stencilSpmvKernel<27, 1><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
-        else stencilSpmvKernel<27, 2><<<g, kReduceThreads, 0, st>>>(a, x, y, w);
+        if (mode == 0) launchChained(stencilSpmvKernel<27, 0>, dim3(g), kReduceThreads, st, a, x, y, w);
+        else if (mode == 1) launchChained(stencilSpmvKernel<27, 1>, dim3(g), kReduceThreads, st, a, x, y, w);
+        else launchChained(stencilSpmvKernel<27, 2>, dim3(g), kReduceThreads, st, a, x, y, w);
     }
     DXG_CUDA(cudaGetLastError());
 }
