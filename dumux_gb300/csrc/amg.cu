@@ -67,9 +67,11 @@ __device__ __forceinline__ void mv(const T* M, const T* v, T* y)
 
 __device__ __forceinline__ void coordOf(int64_t i, int nx, int ny, int& x, int& y, int& z)
 {
-    x = (int)(i % nx);
-    y = (int)((i / nx) % ny);
-    z = (int)(i / ((int64_t)nx * ny));
+    // cell counts fit 32 bits (checked at upload); a 64-bit division would cost more than the row
+    const unsigned q = (unsigned)i / (unsigned)nx;
+    x = (int)((unsigned)i - q * (unsigned)nx);
+    z = (int)(q / (unsigned)ny);
+    y = (int)(q - (unsigned)z * (unsigned)ny);
 }
 
 template <int B, class T>
@@ -272,12 +274,14 @@ __device__ __forceinline__ void restrictCell(const AmgLevel<T>& F, const AmgLeve
     for (int e = 0; e < B; ++e) C.b[i * B + e] = acc[e];
 }
 
-// row i of x = Ainv b on the last level
+// row i of x = Ainv b on the last level (the inverse is stored by columns, so that the threads
+// of consecutive rows read consecutive entries)
 template <class T>
 __device__ __forceinline__ void coarseRow(const AmgLevel<T>& L, int n, int i)
 {
     T t = 0;
-    for (int j = 0; j < n; ++j) t = fma(L.Ainv[(int64_t)i * n + j], L.b[j], t);
+#pragma unroll 8
+    for (int j = 0; j < n; ++j) t = fma(L.Ainv[(int64_t)j * n + i], L.b[j], t);
     L.x[i] = t;
 }
 
@@ -314,67 +318,309 @@ __global__ void amgRestrictKernel(AmgLevel<T> F, AmgLevel<T> C, const KrylovStat
     AMG_LOOP(C) restrictCell<B, DIM, T>(F, C, i);
 }
 
-// The V-cycle below a level of at most kAmgClusterLevel cells as one launch of one thread
-// block cluster: every pass is a loop over the level's cells across the cluster's threads,
-// followed by a cluster barrier (release/acquire at cluster scope orders the passes' global
-// memory traffic).  Same per-cell arithmetic and pass order as the per-level kernels.
+// The V-cycle below a level of at most kAmgClusterLevel cells as one launch of one thread block
+// cluster.  Such a level's passes are a few thousand rows each, so what they cost is the way to
+// the data and the barrier between them (run from global memory, 16 CTAs: ~3 us a pass, 41 us for
+// the levels 2048, 256 and 32 of a 64x64x32 grid; from shared memory 11 us).  So the
+// top level is spread over the CTAs' shared memory -- matrix, pivots, right-hand side and both
+// Jacobi buffers, one thread per row, neighbour rows' values by distributed shared memory -- and
+// the levels below run in CTA 0 alone, out of its shared memory (their matrices too, where they
+// fit) with CTA barriers.  Same per-row arithmetic and pass order as the per-level kernels.
 constexpr int kAmgMaxClusterLevels = 12;
 constexpr int kAmgClusterCtas = 16;
 constexpr int kAmgClusterThreads = 512;
+constexpr size_t kAmgClusterSmem = 220 * 1024;
 template <class T>
 struct AmgCycle {
     AmgLevel<T> lv[kAmgMaxClusterLevels];
     int count;
+    // the level's matrix (last level: the dense inverse) is held in shared memory
+    unsigned char matrixShared[kAmgMaxClusterLevels];
 };
+// Elements of the shared-memory areas: the top level's part of a CTA, then CTA 0's levels with
+// or without their matrices.
+template <int B, int DIM, class T>
+__host__ __device__ inline size_t amgTopElems(int64_t N)
+{
+    constexpr int BB = B * B, S = 2 * DIM + 1;
+    const size_t cpc = (size_t)((N + kAmgClusterCtas - 1) / kAmgClusterCtas);
+    return cpc * (S * BB + BB + 4 * B);
+}
+template <int B, int DIM, class T>
+__host__ __device__ inline size_t amgSubElems(int64_t N, bool last, bool matrix)
+{
+    constexpr int BB = B * B, S = 2 * DIM + 1;
+    const size_t n = (size_t)N * B;
+    if (last) return (matrix ? n * n : 0) + 2 * n;
+    return (size_t)N * ((matrix ? S * BB : 0) + BB + 4 * B);
+}
 
 template <int B, int DIM, class T>
 __global__ void __launch_bounds__(kAmgClusterThreads) amgClusterCycle(AmgCycle<T> cy, const KrylovState* ks)
 {
-    chainWait();
-    if (stopped<T>(ks)) return;   // uniform: the status does not change during the launch
+    constexpr int BB = B * B, S = 2 * DIM + 1;
+    extern __shared__ __align__(16) unsigned char amgRaw[];
     cg::cluster_group cl = cg::this_cluster();
-    const int64_t gid = (int64_t)cl.block_rank() * blockDim.x + threadIdx.x;
-    const int64_t gstride = (int64_t)cl.num_blocks() * blockDim.x;
+    const int rank = (int)cl.block_rank(), tid = (int)threadIdx.x;
     const T omega = (T)kAmgOmega;
-    const T* pre[kAmgMaxClusterLevels];
     const int last = cy.count - 1;
-    for (int l = 0; l < last; ++l) {
-        const AmgLevel<T>& L = cy.lv[l];
-        T* buf[2] = {L.tmp, L.x};
-        int w = 0;
-        for (int64_t i = gid; i < L.N; i += gstride) firstCell<B, T>(L, i, buf[0], omega);
+    const AmgLevel<T>& top = cy.lv[0];
+    const int N = (int)top.N;
+    const int cpc = (N + kAmgClusterCtas - 1) / kAmgClusterCtas;
+
+    // shared memory: this CTA's cells of the top level ...
+    T* As = reinterpret_cast<T*>(amgRaw);      // [S][cpc][BB]
+    T* Ds = As + (size_t)S * cpc * BB;         // [cpc][BB]
+    T* bs = Ds + (size_t)cpc * BB;             // [cpc][B]
+    T* xs = bs + (size_t)cpc * B;              // [2][cpc][B]
+    T* rs = xs + (size_t)2 * cpc * B;          // [cpc][B]
+    const int first = rank * cpc, mine = max(0, min(cpc, N - first));
+    // One decision for the whole cluster: a CTA must not leave while another reads its shared memory.
+    __shared__ int stop;
+    chainWait();
+    if (tid == 0) stop = ks ? __ldcg(&ks->status) != KS_RUNNING : 0;
+    cl.sync();
+    const int stopAll = *cl.map_shared_rank(&stop, 0);
+    if (stopAll) {
         cl.sync();
-        for (int k = 1; k < L.sweeps; ++k, ++w) {
-            for (int64_t i = gid; i < L.N; i += gstride)
-                jacobiCell<B, DIM, T>(L, i, buf[w & 1], nullptr, 0, 0, buf[(w + 1) & 1], omega);
-            cl.sync();
-        }
-        pre[l] = buf[w & 1];
-        for (int64_t i = gid; i < L.N; i += gstride) residualCell<B, DIM, T>(L, i, pre[l]);
-        cl.sync();
-        for (int64_t i = gid; i < cy.lv[l + 1].N; i += gstride) restrictCell<B, DIM, T>(L, cy.lv[l + 1], i);
-        cl.sync();
+        return;
     }
+    // ... and CTA 0's levels below it
+    __shared__ AmgLevel<T> sub[kAmgMaxClusterLevels];
+    __shared__ const T* pre[kAmgMaxClusterLevels];
+    __shared__ int xcAt;       // where level 1's result lies in CTA 0's area
+    auto copy = [&](T* dst, const T* src, size_t k) {
+        constexpr size_t per = 16 / sizeof(T);
+        size_t e0 = 0;
+        if ((((size_t)src | (size_t)dst) & 15) == 0) {
+            e0 = k / per * per;
+            for (size_t e = tid * per; e < e0; e += blockDim.x * per)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + e)),
+                             "l"(src + e) : "memory");
+        }
+        for (size_t e = e0 + tid; e < k; e += blockDim.x) dst[e] = src[e];
+    };
+    if (rank == 0) {
+        T* p = reinterpret_cast<T*>(amgRaw) + (last > 0 ? amgTopElems<B, DIM, T>(N) : 0);
+        auto take = [&](size_t k) {
+            T* q = p;
+            p += k;
+            return q;
+        };
+        for (int l = last > 0 ? 1 : 0; l <= last; ++l) {
+            AmgLevel<T> L = cy.lv[l];
+            const size_t n = (size_t)L.N;
+            if (l == last) {
+                const unsigned m = (unsigned)(n * B);
+                if (cy.matrixShared[l]) {
+                    T* inv = take((size_t)m * m);
+                    copy(inv, cy.lv[l].Ainv, (size_t)m * m);
+                    L.Ainv = inv;
+                }
+                L.b = take(m);
+                if (l > 0) L.x = take(m);
+            } else {
+                if (cy.matrixShared[l]) {
+                    T* m = take(n * S * BB);
+                    copy(m, cy.lv[l].A, n * S * BB);
+                    L.A = m;
+                }
+                T* d = take(n * BB);
+                copy(d, cy.lv[l].Dinv, n * BB);
+                L.Dinv = d;
+                L.b = take(n * B);
+                L.x = take(n * B);
+                L.tmp = take(n * B);
+                L.r = take(n * B);
+            }
+            if (tid == 0) {
+                sub[l] = L;
+                if (l == 1) xcAt = (int)(L.x - reinterpret_cast<T*>(amgRaw));
+            }
+        }
+    }
+    if (last == 0) {
+        // one level only: the direct solve
+        if (rank == 0) {
+            const int n = N * B;
+            __syncthreads();
+            for (int i = tid; i < n; i += blockDim.x) sub[0].b[i] = top.b[i];
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            for (int i = tid; i < n; i += blockDim.x) coarseRow<T>(sub[0], n, i);
+        }
+        cl.sync();
+        return;
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+        copy(As + (size_t)s * cpc * BB, top.A + ((int64_t)s * N + first) * BB, (size_t)mine * BB);
+    copy(Ds, top.Dinv + (int64_t)first * BB, (size_t)mine * BB);
+
+    // this thread's row of the top level and where its neighbours' values are
+    const int lc = tid / B, r = tid % B;
+    const bool row = lc < mine;
+    int x = 0, y = 0, z = 0;
+    if (row) coordOf(first + lc, top.nx, top.ny, x, y, z);
+    const T* nb[S];            // the neighbours' entries in Jacobi buffer 0
+    int agg[S];                // the neighbours' aggregates
+    unsigned has = 0;
+    const AmgLevel<T>& C1 = cy.lv[1];
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        int64_t d = 0;
+        const bool ok = row && (s == DIM || neighbour<DIM>(s, x, y, z, top.nx, top.ny, top.nz, &d));
+        const int j = ok ? first + lc + (int)d : first;
+        const int axis = s < DIM ? DIM - 1 - s : s - DIM - 1, sg = s < DIM ? -1 : 1;
+        const int jx = x + (s != DIM && axis == 0 ? sg : 0), jy = y + (s != DIM && axis == 1 ? sg : 0),
+                  jz = z + (s != DIM && axis == 2 ? sg : 0);
+        agg[s] = ok ? (jx >> 1) + C1.nx * ((jy >> 1) + C1.ny * (jz >> 1)) : 0;
+        const int owner = j / cpc;
+        nb[s] = cl.map_shared_rank(xs, owner) + (size_t)(j - owner * cpc) * B;
+        has |= ok ? 1u << s : 0u;
+    }
+    const T* xc = nullptr;     // the coarse correction, in CTA 0
+    // row r of A x~, x~ the values of Jacobi buffer w (plus the prolongated correction)
+    auto rowTop = [&](int w) -> T {
+        T out = 0;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            if (!((has >> s) & 1u)) continue;
+            const T* q = nb[s] + (size_t)w * cpc * B;
+            T v[B];
+#pragma unroll
+            for (int e = 0; e < B; ++e) v[e] = q[e];
+            if (xc)
+#pragma unroll
+                for (int e = 0; e < B; ++e) v[e] += xc[agg[s] * B + e];
+            const T* m = As + ((size_t)s * cpc + lc) * BB + r * B;
+            T t = m[0] * v[0];
+#pragma unroll
+            for (int e = 1; e < B; ++e) t = fma(m[e], v[e], t);
+            out += t;
+        }
+        return out;
+    };
+    // row r of D^-1 times the cell's values, this row's in `own`
+    auto rowPivot = [&](T own) -> T {
+        T v[B];
+        v[0] = own;
+        if constexpr (B == 2) {
+            const T other = __shfl_xor_sync(0xffffffffu, own, 1);
+            v[0] = r == 0 ? own : other;
+            v[1] = r == 0 ? other : own;
+        }
+        const T* m = Ds + (size_t)(row ? lc : 0) * BB + r * B;
+        T t = m[0] * v[0];
+#pragma unroll
+        for (int e = 1; e < B; ++e) t = fma(m[e], v[e], t);
+        return t;
+    };
+    auto jacobiTop = [&](int w, T* out) {
+        T res = 0;
+        if (row) res = bs[lc * B + r] - rowTop(w);
+        const T yv = rowPivot(res);
+        if (row) {
+            T xi = xs[((size_t)w * cpc + lc) * B + r];
+            if (xc) xi += xc[agg[DIM] * B + r];
+            out[lc * B + r] = xi + omega * yv;
+        }
+    };
+    for (int e = tid; e < mine * B; e += blockDim.x) bs[e] = top.b[(int64_t)first * B + e];
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    // down on the top level: sweeps alternate between the buffers
     {
-        const AmgLevel<T>& L = cy.lv[last];
-        const int n = (int)L.N * B;
-        for (int64_t i = gid; i < n; i += gstride) coarseRow<T>(L, n, (int)i);
+        const T yv = rowPivot(row ? bs[lc * B + r] : T(0));
+        if (row) xs[lc * B + r] = omega * yv;
+    }
+    cl.sync();
+    int w = 0;
+    for (int k = 1; k < top.sweeps; ++k, w ^= 1) {
+        jacobiTop(w, xs + (size_t)(w ^ 1) * cpc * B);
         cl.sync();
     }
-    for (int l = last - 1; l >= 0; --l) {
-        const AmgLevel<T>& L = cy.lv[l];
-        const AmgLevel<T>& C = cy.lv[l + 1];
-        T* buf[2] = {L.tmp, L.x};
-        int w = L.sweeps - 1;   // index of the last pre-smoothing write
-        for (int64_t i = gid; i < L.N; i += gstride)
-            jacobiCell<B, DIM, T>(L, i, pre[l], C.x, C.nx, C.ny, buf[(w + 1) & 1], omega);
-        ++w;
-        cl.sync();
-        for (int k = 1; k < L.sweeps; ++k, ++w) {
-            for (int64_t i = gid; i < L.N; i += gstride)
-                jacobiCell<B, DIM, T>(L, i, buf[w & 1], nullptr, 0, 0, buf[(w + 1) & 1], omega);
-            cl.sync();
+    if (row) rs[lc * B + r] = bs[lc * B + r] - rowTop(w);
+    cl.sync();
+
+    if (rank == 0) {
+        // restriction from the CTAs' residuals (the aggregate's cells in fixed order) ...
+        for (int i = tid; i < (int)C1.N; i += blockDim.x) {
+            int cx, cy_, cz;
+            coordOf(i, C1.nx, C1.ny, cx, cy_, cz);
+            T acc[B];
+#pragma unroll
+            for (int e = 0; e < B; ++e) acc[e] = 0;
+            for (int dz = 0; dz < (DIM == 3 ? 2 : 1); ++dz) {
+                if (2 * cz + dz >= top.nz) continue;
+                for (int dy = 0; dy < 2; ++dy) {
+                    if (2 * cy_ + dy >= top.ny) continue;
+                    for (int dx = 0; dx < 2; ++dx) {
+                        if (2 * cx + dx >= top.nx) continue;
+                        const int f = 2 * cx + dx + top.nx * (2 * cy_ + dy + top.ny * (2 * cz + dz));
+                        const int owner = f / cpc;
+                        const T* q = cl.map_shared_rank(rs, owner) + (size_t)(f - owner * cpc) * B;
+#pragma unroll
+                        for (int e = 0; e < B; ++e) acc[e] += q[e];
+                    }
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < B; ++e) sub[1].b[i * B + e] = acc[e];
         }
+        __syncthreads();
+        // ... and the cycle below
+        for (int l = 1; l < last; ++l) {
+            const AmgLevel<T>& L = sub[l];
+            T* buf[2] = {L.tmp, L.x};
+            int v = 0;
+            for (int i = tid; i < (int)L.N; i += blockDim.x) firstCell<B, T>(L, i, buf[0], omega);
+            __syncthreads();
+            for (int k = 1; k < L.sweeps; ++k, ++v) {
+                for (int i = tid; i < (int)L.N; i += blockDim.x)
+                    jacobiCell<B, DIM, T>(L, i, buf[v & 1], nullptr, 0, 0, buf[(v + 1) & 1], omega);
+                __syncthreads();
+            }
+            if (tid == 0) pre[l] = buf[v & 1];
+            for (int i = tid; i < (int)L.N; i += blockDim.x) residualCell<B, DIM, T>(L, i, buf[v & 1]);
+            __syncthreads();
+            for (int i = tid; i < (int)sub[l + 1].N; i += blockDim.x) restrictCell<B, DIM, T>(L, sub[l + 1], i);
+            __syncthreads();
+        }
+        {
+            const AmgLevel<T>& L = sub[last];
+            const int n = (int)L.N * B;
+            for (int i = tid; i < n; i += blockDim.x) coarseRow<T>(L, n, i);
+            __syncthreads();
+        }
+        for (int l = last - 1; l >= 1; --l) {
+            const AmgLevel<T>& L = sub[l];
+            const AmgLevel<T>& C = sub[l + 1];
+            T* buf[2] = {L.tmp, L.x};
+            int v = L.sweeps - 1;   // index of the last pre-smoothing write
+            for (int i = tid; i < (int)L.N; i += blockDim.x)
+                jacobiCell<B, DIM, T>(L, i, pre[l], C.x, C.nx, C.ny, buf[(v + 1) & 1], omega);
+            ++v;
+            __syncthreads();
+            for (int k = 1; k < L.sweeps; ++k, ++v) {
+                for (int i = tid; i < (int)L.N; i += blockDim.x)
+                    jacobiCell<B, DIM, T>(L, i, buf[v & 1], nullptr, 0, 0, buf[(v + 1) & 1], omega);
+                __syncthreads();
+            }
+        }
+    }
+    cl.sync();
+    // up: the correction out of CTA 0 into the first sweep; the last one writes the result
+    xc = cl.map_shared_rank(reinterpret_cast<T*>(amgRaw), 0) + *cl.map_shared_rank(&xcAt, 0);
+    T* const result = top.x + (int64_t)first * B;
+    jacobiTop(w, top.sweeps > 1 ? xs + (size_t)(w ^ 1) * cpc * B : result);
+    w ^= 1;
+    cl.sync();
+    xc = nullptr;
+    for (int k = 1; k < top.sweeps; ++k, w ^= 1) {
+        const bool end = k + 1 == top.sweeps;
+        jacobiTop(w, end ? result : xs + (size_t)(w ^ 1) * cpc * B);
+        cl.sync();
     }
 }
 
@@ -463,7 +709,7 @@ __device__ void coarseInvertCta(const AmgLevel<T>& L, int* singular, unsigned ch
             }
         __syncthreads();
     }
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) L.Ainv[e] = a[e];
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) L.Ainv[e] = a[e % n * n + e / n];   // by columns
 }
 
 template <int B, int DIM, class T>
@@ -531,16 +777,33 @@ int64_t vcycle(const std::vector<AmgLevel<T>>& Ls, size_t l, const KrylovState* 
 {
     const AmgLevel<T>& L = Ls[l];
     const unsigned g = gridFor(L.N);
+    size_t elems = 0;
     if (L.N <= kAmgClusterLevel && Ls.size() - l <= (size_t)kAmgMaxClusterLevels) {
+        const size_t last = Ls.size() - 1;
+        elems = last > l ? amgTopElems<B, DIM, T>(L.N) : 0;
+        for (size_t k = last > l ? l + 1 : l; k <= last; ++k) elems += amgSubElems<B, DIM, T>(Ls[k].N, k == last, false);
+        if (elems * sizeof(T) > kAmgClusterSmem) elems = 0;   // long thin grids: from a level further down
+    }
+    if (elems > 0) {
         // this level and all below: one cluster launch
         AmgCycle<T> cy{};
         cy.count = (int)(Ls.size() - l);
         for (int k = 0; k < cy.count; ++k) cy.lv[k] = Ls[l + k];
+        // the matrices of the levels below, the coarsest first, while they fit
+        for (int k = cy.count - 1; k >= (cy.count > 1 ? 1 : 0); --k) {
+            const size_t more = amgSubElems<B, DIM, T>(cy.lv[k].N, k + 1 == cy.count, true) -
+                                amgSubElems<B, DIM, T>(cy.lv[k].N, k + 1 == cy.count, false);
+            if ((elems + more) * sizeof(T) > kAmgClusterSmem) break;
+            cy.matrixShared[k] = 1;
+            elems += more;
+        }
         auto kern = amgClusterCycle<B, DIM, T>;
         DXG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        DXG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAmgClusterSmem));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kAmgClusterCtas);
         cfg.blockDim = dim3(kAmgClusterThreads);
+        cfg.dynamicSmemBytes = elems * sizeof(T);
         cfg.stream = st;
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
