@@ -31,6 +31,7 @@ UNITS = {
     "amg.cu": [],
     "mpfa.cu": ["--fmad=false"],
     "stencilwave.cu": [],
+    "stencilpack.cu": [],
     "stencillane.cu": [],
     "linesweep.cu": [],
 }

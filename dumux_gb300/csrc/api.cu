@@ -596,6 +596,7 @@ void tabulate(dxg_ctx* c, const dxg_problem_desc* d)
     c->laneHandoff.release();
     c->laneHandoffBytes = 0;
     c->packPlan = LanePackPlan{};
+    c->stencilPack = StencilPackPlan{};
     c->packPlanned = false;
     c->packMem.release();
     c->waveTuneCount = 0;
@@ -765,6 +766,7 @@ void tabulateMpfa(dxg_ctx* c, const dxg_problem_desc* d)
     c->laneHandoff.release();
     c->laneHandoffBytes = 0;
     c->packPlan = LanePackPlan{};
+    c->stencilPack = StencilPackPlan{};
     c->packPlanned = false;
     c->packMem.release();
     c->waveTuneCount = 0;
@@ -926,7 +928,9 @@ MpfaArgs mpfaArgs(const dxg_ctx* c)
     return a;
 }
 
-// The MPFA-O preconditioner apply: 1 the one-CTA line sweeps (2D with up to 1024 lines:
+// The MPFA-O preconditioner apply: 4 the line sweeps over packed records (2D, one unknown: auto
+// wherever their plan fits; 256 x 256: 0.30 ms per apply against 0.667 ms for kind 1), 1 the
+// one-CTA line sweeps (2D with up to 1024 lines:
 // DXG_ILU_WAVEFRONT or auto), 2 the cluster line sweeps (2D: DXG_ILU_LANES, or auto beyond
 // 1024 lines), 3 the 3D cluster sweeps (one z-plane per CTA: DXG_ILU_LANES or auto), 0 the
 // level-by-level kernel (DXG_ILU_LEVELS, or when none fits).  On 256 x 256 the one-CTA sweeps
@@ -939,7 +943,7 @@ int mpfaSweep(const dxg_ctx* c, const StencilArgs& sa)
     case DXG_ILU_LEVELS: return 0;
     case DXG_ILU_LANES: return lanes ? 2 : lanes3 ? 3 : 0;
     case DXG_ILU_WAVEFRONT: return wave ? 1 : 0;
-    default: return wave ? 1 : lanes ? 2 : lanes3 ? 3 : 0;
+    default: return c->stencilPack.ok ? 4 : wave ? 1 : lanes ? 2 : lanes3 ? 3 : 0;
     }
 }
 
@@ -965,6 +969,10 @@ StencilArgs stencilArgs(dxg_ctx* c)
     std::memcpy(a.tri, c->mpTri, sizeof(a.tri));
     a.err = c->singular.get() + 1;
     a.waitNs = c->waitNs;
+    if (c->packMem.get() && c->stencilPack.ok) {
+        a.pack[0] = c->packMem.get();
+        a.pack[1] = a.pack[0] + stencilPackBytes(c->stencilPack, 1);
+    }
     return a;
 }
 
@@ -1195,6 +1203,23 @@ void preparePack(dxg_ctx* c)
         return;
     }
     DXG_CUDA(cudaMemsetAsync(c->packMem.get() + records, 0xff, handoff, c->stream));
+}
+
+// As preparePack, for the scalar 2D MPFA-O stencil.
+void prepareStencilPack(dxg_ctx* c)
+{
+    if (!c->packPlanned) {
+        c->packPlanned = true;
+        c->stencilPack = makeStencilPackPlan(stencilArgs(c));
+    }
+    if (!c->stencilPack.ok || c->packMem.get()) return;
+    try {
+        c->packMem.alloc(stencilPackBytes(c->stencilPack, 1) + stencilPackBytes(c->stencilPack, -1));
+    } catch (const Error& e) {
+        if (e.status != DXG_ERR_OOM) throw;
+        cudaGetLastError();
+        c->stencilPack.ok = false;
+    }
 }
 
 template <class T>
@@ -1435,6 +1460,11 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
             if constexpr (!mixed) {
                 launchStencilFactor(stencilArgs(c), st);
                 c->launches += 1;
+                prepareStencilPack(c);
+                if (c->stencilPack.ok) {   // whatever kernel is set: it may be changed without a new factor
+                    launchStencilPack(stencilArgs(c), c->stencilPack, st);
+                    c->launches += 1;
+                }
             }
         } else if (c->linearSolver == DXG_LINEAR_SOLVER_AMG_BICGSTAB) {
             // AMG setup: fine pivots, then each coarse operator (with its pivots) from the one above
@@ -1505,6 +1535,7 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
             if (c->mpfa) {
                 TimedScope ts(c, DXG_KC_ILU_SWEEP, c->bytesSweep);
                 switch (mpfaSweep(c, sa)) {
+                case 4: launchStencilPackApply(sa, c->stencilPack, in, yOut, st); return 1;
                 case 3: launchStencilLane3d(sa, in, yOut, st); return 2;
                 case 2: launchStencilLane2d(sa, in, yOut, st); return 2;
                 case 1: launchStencilWave2d(sa, in, yOut, st); return 2;
@@ -1603,7 +1634,7 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
         // a sweep that gave up may leave hand-off entries written: start the next from scratch
         if (c->laneHandoffBytes)
             DXG_CUDA(cudaMemsetAsync(c->laneHandoff.get(), 0xff, c->laneHandoffBytes, st));
-        if (c->packMem.get()) {
+        if (c->packMem.get() && c->packPlan.ok) {
             const size_t ts = sizeof(PT), handoff = laneHandoffBytes(c->packPlan, ts);
             DXG_CUDA(cudaMemsetAsync(c->packMem.get() + c->packMem.bytes() - handoff, 0xff, handoff, st));
         }
@@ -2202,6 +2233,8 @@ int dxg_describe(const dxg_ctx* c, char* buf, int64_t len)
                             std::to_string(sa.nz) + " CTAs"
                : k == 2 ? "line sweeps (one thread per grid line, levels x+2y) over a cluster of " +
                             std::to_string((sa.ny + 127) / 128) + " CTAs"
+               : k == 4 ? "line sweeps over packed records (one lane per grid line, levels x+2y) over a cluster of " +
+                            std::to_string(c->stencilPack.ctas) + " CTAs"
                : k == 1 ? "line sweeps (one thread per grid line, levels x+2y) in one CTA"
                         : "hyperplanes x+2y+4z level by level in one CTA");
     }

@@ -121,6 +121,7 @@ struct dxg_ctx {
     // lane sweeps over packed records (lanepack.cu): the default natural-order apply wherever their
     // plan fits; planned at the first factorisation that uses them
     dxg::LanePackPlan packPlan;
+    dxg::StencilPackPlan stencilPack;     // ... and of the 2D scalar MPFA-O stencil
     bool packPlanned = false;
     dxg::DevBuf<unsigned char> packMem;   // records of both sweeps, then the hand-off buffer
     dxg::DevBuf<unsigned char> laneHandoff;

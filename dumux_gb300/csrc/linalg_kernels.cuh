@@ -141,7 +141,17 @@ struct StencilArgs {
     int8_t tri[104][3] = {};
     int* err = nullptr;                    // DXG_ERR_TIMEOUT of a sweep that gave up waiting
     unsigned long long waitNs = 0;         // wait limit of the cluster sweeps (0: 0.5 s)
+    unsigned char* pack[2] = {};           // packed records of the forward / backward sweep (stencilpack.cu)
 };
+// Sweeps of the scalar 2D 9-point stencil over packed records (stencilpack.cu), one cluster.
+struct StencilPackPlan {
+    bool ok = false;
+    int warps = 0, ctas = 0, steps = 0, stages = 0;   // warps per CTA, padded steps per warp, ring depth
+};
+StencilPackPlan makeStencilPackPlan(const StencilArgs& a);
+size_t stencilPackBytes(const StencilPackPlan& p, int dir);
+void launchStencilPack(const StencilArgs& a, const StencilPackPlan& p, cudaStream_t st);
+void launchStencilPackApply(const StencilArgs& a, const StencilPackPlan& p, const double* d, double* v, cudaStream_t st);
 void launchStencilSpmv(const StencilArgs& a, const double* x, double* y, const double* w, int mode, cudaStream_t st);
 void launchStencilFactor(const StencilArgs& a, cudaStream_t st);
 // the preconditioner apply: the level-by-level kernel (any stencil), the one-CTA line sweeps

@@ -65,3 +65,30 @@ def test_packed_lane_sweeps_wait_limit_expires_and_the_context_recovers():
     again = ctx.linear_solve(1e-10, 500)
     assert again["converged"] and again["iterations"] == first["iterations"]
     assert np.array_equal(ctx.update(), x0)
+
+
+# two warps of 32 lines per CTA (one on long lines); histories across warps, CTAs and remainders
+@pytest.mark.parametrize("cells", [(1, 1), (5, 4), (9, 31), (3, 33), (70, 64), (6, 65), (40, 130), (33, 257), (300, 40)])
+def test_packed_mpfa_sweeps_equal_level_kernel(cells):
+    desc, u, _ = problems.mpfa_linear_field_problem(cells=cells, spacing_seed=3)
+    n0, x0, _ = _solve(desc, u, u, "levels", "fp64", 0.0)
+    n1, x1, how = _solve(desc, u, u, "auto", "fp64", 0.0)
+    assert "packed records" in how
+    assert n1 == n0
+    assert np.array_equal(x1, x0)
+
+
+def test_packed_mpfa_sweeps_wait_limit_expires_and_the_context_recovers():
+    desc, u, _ = problems.mpfa_linear_field_problem(cells=(64, 192), spacing_seed=3)
+    ctx = Context(desc)
+    ctx.set_solution(u)
+    ctx.assemble_jacobian_and_residual()
+    first = ctx.linear_solve(1e-10, 500)
+    assert first["converged"] and "packed records" in ctx.describe()
+    x0 = ctx.update()
+    ctx.set_wait_limit(1e-6)
+    with pytest.raises(Exception, match="timed out"):
+        ctx.linear_solve(1e-10, 500)
+    ctx.set_wait_limit(0.5)
+    assert ctx.linear_solve(1e-10, 500)["iterations"] == first["iterations"]
+    assert np.array_equal(ctx.update(), x0)
