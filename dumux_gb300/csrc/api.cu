@@ -1151,35 +1151,6 @@ bool usePack(const dxg_ctx* c)
            (c->iluKernel == DXG_ILU_LANES || c->iluKernel == DXG_ILU_AUTO);
 }
 
-template <class T>
-LanePackArgs<T> packArgs(dxg_ctx* c, const T* A, const T* L, const T* Dinv, const T* rhs, T* v)
-{
-    const LanePackPlan& p = c->packPlan;
-    LanePackArgs<T> a{};
-    a.nx = c->pcHost.nx;
-    a.ny = c->pcHost.ny;
-    a.nz = c->dim == 3 ? c->pcHost.nz : 1;
-    a.N = c->N;
-    a.nyb = p.nyb;
-    a.warps = p.warps;
-    a.steps = p.steps;
-    a.stages = p.stages;
-    a.ctas = p.ctas;
-    a.clusterSize = p.clusterSize;
-    a.Lf = L;
-    a.A = A;
-    a.Dinv = Dinv;
-    a.pack[0] = c->packMem.get();
-    a.pack[1] = a.pack[0] + lanePackBytes(p, 1, sizeof(T));
-    a.handoff = reinterpret_cast<T*>(a.pack[1] + lanePackBytes(p, -1, sizeof(T)));
-    a.rhs = rhs;
-    a.v = v;
-    a.err = c->singular.get() + 1;
-    a.ks = c->ks.get();
-    a.waitNs = c->waitNs ? c->waitNs : 500000000ull;
-    return a;
-}
-
 // Before a factorisation: plans the packed sweeps and makes their buffers on first use.  Where
 // the records do not fit into device memory the context goes on without them.
 template <class T>

@@ -160,6 +160,7 @@ struct Slot {
     double reduction = 0.0, lastReduction = 1.0, initialResidual = 0.0;
     // linear solve of the current iteration
     bool solving = false, linConv = false;
+    bool packed = false;              // the packed records hold the current factor
     int chunks = 0, linIters = 0;
     int linStatus = DXG_OK;
     // outcome
@@ -189,6 +190,8 @@ struct dxg_batch {
     bool redBlack = false;            // red-black ordered ILU(0) instead of the natural order
     bool amg = false;                 // AMG-BiCGSTAB instead of ILU(0)-BiCGSTAB
     int64_t budget = 0, bytesInUse = 0;
+    int64_t packBytes = 0;            // packed factor records of the members (extra to bytesInUse)
+    bool noPacks = false;             // the device memory did not hold them
     int64_t nextId = 1;
     int64_t launches = 0;
     std::map<int64_t, std::unique_ptr<Slot>> slots;
@@ -467,12 +470,12 @@ BicgArgs<double> krylovArgs(dxg_ctx* c, bool mixed)
 // The sweeps read the members' preconditioner inputs and write only their
 // preconditioner outputs, which hold no state between BiCGSTAB half steps.
 template <class PT>
-WaveBatchPlan tunePlan(dxg_batch* B, const Members& S, int dim, int b)
+WaveBatchPlan tunePlan(dxg_batch* B, const Members& S, int dim, int b, bool tune)
 {
     const bool fp64 = sizeof(PT) == 8;
     std::vector<WaveBatchPlan> cand = candidates(S, dim, b, fp64);
     if (cand.empty()) throw Error(DXG_ERR_ARG, "no batched ILU(0) sweep shape fits these grids");
-    if (!B->autotune || cand.size() == 1) {
+    if (!tune || cand.size() == 1) {
         // fixed rule: the largest cluster with the fewest threads and the deepest prefetch
         WaveBatchPlan best = cand.front();
         for (const auto& p : cand)
@@ -556,9 +559,9 @@ TuneCache& tuneCache()
 }
 
 template <class PT>
-WaveBatchPlan planFor(dxg_batch* B, const Members& S, int dim, int b)
+WaveBatchPlan planFor(dxg_batch* B, const Members& S, int dim, int b, bool tune)
 {
-    const auto key = std::make_tuple(B->device, (int)B->autotune, shapeKey(S, dim, b, (int)sizeof(PT)));
+    const auto key = std::make_tuple(B->device, (int)tune, shapeKey(S, dim, b, (int)sizeof(PT)));
     TuneCache& tc = tuneCache();
     {
         std::lock_guard<std::mutex> lock(tc.m);
@@ -568,7 +571,7 @@ WaveBatchPlan planFor(dxg_batch* B, const Members& S, int dim, int b)
             if (completeWaveBatchPlan(p, geomsFor(S, p.ctas), dim, b, sizeof(PT) == 8) > 0) return p;
         }
     }
-    WaveBatchPlan p = tunePlan<PT>(B, S, dim, b);
+    WaveBatchPlan p = tunePlan<PT>(B, S, dim, b, tune);
     std::lock_guard<std::mutex> lock(tc.m);
     tc.plans[key] = p;
     return p;
@@ -604,6 +607,18 @@ struct GroupState {
     std::vector<SweepClass> classes;
     std::vector<int> classOf;       // per member: index into classes
     std::vector<WaveGeom> geo;      // per member, from its class's launch shape
+    // packed sweeps instead of the classes' (which then only factorise): launches that follow one
+    // another, each of members whose clusters are resident together
+    struct PackRound {
+        const uint2* map;
+        unsigned blocks;
+    };
+    bool packs = false;
+    std::vector<PackRound> rounds;
+    int packWarps = 0;
+    size_t packSmem = 0;
+    const void* dPkP = nullptr;      // LanePackArgs<PT> applied to p / to r
+    const void* dPkR = nullptr;
     DevBuf<unsigned char> args;
     const BicgArgs<double>* dBicg = nullptr;
     const void* dSv1 = nullptr;      // SpmvArgs<double, double, PT>
@@ -840,20 +855,113 @@ std::vector<AmgPassList<PT>> amgCycleSchedule(const std::vector<std::vector<AmgL
     return out;
 }
 
+// Gives back the members' packed records; the groups are rebuilt without or with new ones.
+void dropPacks(dxg_batch* B)
+{
+    if (B->packBytes == 0) return;
+    DXG_CUDA(cudaStreamSynchronize(B->stream));
+    B->groups.clear();
+    for (auto& kv : B->slots) {
+        kv.second->c->packMem.release();
+        kv.second->packed = false;
+    }
+    B->packBytes = 0;
+}
+
+// Whether a group's natural-order sweeps run over packed records: every member's plan fits, and
+// device memory (or the batch's budget) holds the records beside the problems.  Their buffers are
+// made here.  One launch of the packed sweeps does both directions of several problems: an ensemble
+// of twelve grids of 16 to 40 cells a side takes 0.45 s in FP32 against 0.68 s on the cluster
+// wavefront (six in FP64 0.44 against 0.94 s), twelve of 16 to 22 cells 0.11 against 0.15 s.
+template <class PT>
+bool preparePacks(dxg_batch* B, const Members& S)
+{
+    if (B->noPacks) return false;
+    int warps = 0;
+    size_t smem = 0;
+    int64_t need = 0;
+    auto bytesOf = [](const LanePackPlan& p) {
+        return lanePackBytes(p, 1, sizeof(PT)) + lanePackBytes(p, -1, sizeof(PT)) + laneHandoffBytes(p, sizeof(PT));
+    };
+    for (Slot* s : S) {
+        dxg_ctx* c = s->c;
+        if (!c->packPlanned) {
+            c->packPlanned = true;
+            c->packPlan = makeLanePackBatchPlan<PT>(c->dim, c->pcHost.nx, c->pcHost.ny, c->dim == 3 ? c->pcHost.nz : 1, c->b);
+        }
+        if (!c->packPlan.ok) return false;
+        warps = std::max(warps, c->packPlan.warps);
+        smem = std::max(smem, lanePackSmem<PT>(c->packPlan));
+        if (!c->packMem.get()) need += bytesOf(c->packPlan);
+    }
+    const int resident = lanePackResident<PT>(S[0]->c->packPlan, warps, smem);
+    for (Slot* s : S)
+        if (s->c->packPlan.grid / kLanePackBatchCluster > resident) return false;
+    if (B->budget > 0 && B->bytesInUse + B->packBytes + need > B->budget) return false;
+    for (Slot* s : S) {
+        dxg_ctx* c = s->c;
+        if (c->packMem.get()) continue;
+        const size_t bytes = bytesOf(c->packPlan), handoff = laneHandoffBytes(c->packPlan, sizeof(PT));
+        try {
+            c->packMem.alloc(bytes);
+        } catch (const Error& e) {
+            if (e.status != DXG_ERR_OOM) throw;
+            cudaGetLastError();
+            dropPacks(B);
+            B->noPacks = true;
+            return false;
+        }
+        B->packBytes += (int64_t)bytes;
+        DXG_CUDA(cudaMemsetAsync(c->packMem.get() + bytes - handoff, 0xff, handoff, B->stream));
+    }
+    return true;
+}
+template <class PT>
+void packFactor(dxg_batch* B, Slot* s)
+{
+    dxg_ctx* c = s->c;
+    launchLanePack<PT>(c->packPlan, packArgs<PT>(c, Pre<PT>::A(c), Pre<PT>::L(c), Pre<PT>::Dinv(c), nullptr, nullptr),
+                       B->stream);
+    B->launches += 1;
+    s->packed = true;
+}
+// Which members share a launch: first fit over the members by falling length of their sweeps.
+template <class PT>
+std::vector<std::vector<uint2>> packRounds(const Members& S, int warps, size_t smem)
+{
+    const int room = lanePackResident<PT>(S[0]->c->packPlan, warps, smem) * kLanePackBatchCluster;
+    std::vector<int> order(S.size());
+    for (size_t k = 0; k < S.size(); ++k) order[k] = (int)k;
+    auto length = [&](int k) { return S[k]->c->packPlan.steps + (S[k]->c->dim == 3 ? S[k]->c->pcHost.nz : 0); };
+    std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return length(p) > length(q); });
+    std::vector<std::vector<uint2>> rounds;
+    for (int k : order) {
+        const int grid = S[k]->c->packPlan.grid;
+        size_t r = 0;
+        while (r < rounds.size() && (int)rounds[r].size() + grid > room) ++r;
+        if (r == rounds.size()) rounds.emplace_back();
+        for (int j = 0; j < grid; ++j) rounds[r].push_back(make_uint2((unsigned)k, (unsigned)j));
+    }
+    return rounds;
+}
+
 // (Re)builds the group's chunk arguments when its membership changed.
 template <class PT>
 GroupState& groupState(dxg_batch* B, const GroupKey& key, const Members& S)
 {
-    auto& slot = B->groups[key];
     std::vector<int64_t> ids;
     for (Slot* s : S) ids.push_back(s->id);
-    if (slot && slot->ids == ids) return *slot;
+    const auto known = B->groups.find(key);
+    if (known != B->groups.end() && known->second->ids == ids) return *known->second;
+    const bool packs = !B->redBlack && !B->amg && preparePacks<PT>(B, S);
+    auto& slot = B->groups[key];
     constexpr bool mixed = sizeof(PT) == 4;
     cudaStream_t st = B->stream;
     DXG_CUDA(cudaStreamSynchronize(st));     // the previous arguments may still be read
     slot.reset(new GroupState());
     GroupState& G = *slot;
     G.ids = ids;
+    G.packs = packs;
     const int n = (int)S.size();
     const int dim = S[0]->c->dim, b = S[0]->c->b;
     if (!B->redBlack && !B->amg) {
@@ -872,9 +980,9 @@ GroupState& groupState(dxg_batch* B, const GroupKey& key, const Members& S)
         for (SweepClass& sc : G.classes) {
             Members sub;
             for (int k : sc.members) sub.push_back(S[k]);
-            sc.plan = planFor<PT>(B, sub, dim, b);
+            sc.plan = planFor<PT>(B, sub, dim, b, B->autotune && !packs);
         }
-        refineClassPlans<PT>(B, G.classes, S, dim, b);
+        if (!packs) refineClassPlans<PT>(B, G.classes, S, dim, b);
         for (SweepClass& sc : G.classes) {
             Members sub;
             for (int k : sc.members) sub.push_back(S[k]);
@@ -893,6 +1001,7 @@ GroupState& groupState(dxg_batch* B, const GroupKey& key, const Members& S)
     std::vector<BicgArgs<double>> ba(n);
     std::vector<SpmvArgs<double, double, PT>> sv1(n), sv2(n);
     std::vector<WaveArgs<PT>> fwP(n), fwR(n), bw(n);   // member order; repacked per class below
+    std::vector<LanePackArgs<PT>> pkP, pkR;
     std::vector<RbArgs<PT>> rbP(n), rbR(n);
     std::vector<ToDoubleArgs> td(n);
     for (int k = 0; k < n; ++k) {
@@ -913,7 +1022,13 @@ GroupState& groupState(dxg_batch* B, const GroupKey& key, const Members& S)
         sv.w = ba[k].r;
         sv2[k] = sv;
         const PT* PA = Pre<PT>::A(c);
-        if (!B->redBlack && !B->amg) {
+        if (packs) {
+            if (S[k]->solving && !S[k]->packed) packFactor<PT>(B, S[k]);
+            pkP.push_back(packArgs<PT>(c, PA, Pre<PT>::L(c), Pre<PT>::Dinv(c), Pre<PT>::pIn(c), Pre<PT>::yOut(c)));
+            pkR.push_back(packArgs<PT>(c, PA, Pre<PT>::L(c), Pre<PT>::Dinv(c), Pre<PT>::rIn(c), Pre<PT>::yOut(c)));
+            G.packWarps = std::max(G.packWarps, c->packPlan.warps);
+            G.packSmem = std::max(G.packSmem, lanePackSmem<PT>(c->packPlan));
+        } else if (!B->redBlack && !B->amg) {
             fwP[k] = waveArgsOf<PT>(c, G.geo[k], PA, Pre<PT>::L(c), Pre<PT>::Dinv(c), Pre<PT>::pIn(c),
                                     Pre<PT>::yOut(c), c->ks.get());
             fwR[k] = waveArgsOf<PT>(c, G.geo[k], PA, Pre<PT>::L(c), Pre<PT>::Dinv(c), Pre<PT>::rIn(c),
@@ -964,8 +1079,17 @@ GroupState& groupState(dxg_batch* B, const GroupKey& key, const Members& S)
         for (auto& pl : amgCycleSchedule<PT>(lr, ks, b))
             amgOffR.push_back({pl.kind, pack(host, pl.passes), pack(host, pl.map), (unsigned)pl.map.size()});
     }
+    size_t oPP = 0, oPR = 0;
+    std::vector<std::pair<size_t, unsigned>> oRounds;
+    if (packs) {
+        oPP = pack(host, pkP);
+        oPR = pack(host, pkR);
+        for (const auto& r : packRounds<PT>(S, G.packWarps, G.packSmem))
+            oRounds.push_back({pack(host, r), (unsigned)r.size()});
+    }
     std::vector<std::array<size_t, 3>> oc;
     for (const SweepClass& sc : G.classes) {
+        if (packs) break;
         std::vector<WaveArgs<PT>> cP, cR, cW;
         for (int k : sc.members) {
             cP.push_back(fwP[k]);
@@ -980,7 +1104,10 @@ GroupState& groupState(dxg_batch* B, const GroupKey& key, const Members& S)
     G.dBicg = reinterpret_cast<const BicgArgs<double>*>(d + oB);
     G.dSv1 = d + o1;
     G.dSv2 = d + o2;
-    for (size_t q = 0; q < G.classes.size(); ++q) {
+    G.dPkP = d + oPP;
+    G.dPkR = d + oPR;
+    for (const auto& r : oRounds) G.rounds.push_back({reinterpret_cast<const uint2*>(d + r.first), r.second});
+    for (size_t q = 0; q < oc.size(); ++q) {
         G.classes[q].dFwP = d + oc[q][0];
         G.classes[q].dFwR = d + oc[q][1];
         G.classes[q].dBw = d + oc[q][2];
@@ -1017,6 +1144,13 @@ void enqueueChunk(dxg_batch* B, const GroupState& G, int n, int dim, int b)
         if (B->redBlack) {
             TimedB tb(B, DXG_KC_ILU_SWEEP, G.sweepBytes);
             launchRbApplyBatch<PT>(static_cast<const RbArgs<PT>*>(onP ? G.dRbP : G.dRbR), G.mapH, b, dim, st);
+            return;
+        }
+        if (G.packs) {
+            TimedB tb(B, DXG_KC_ILU_SWEEP, G.sweepBytes);
+            for (const GroupState::PackRound& r : G.rounds)
+                launchLanePackApplyBatch<PT>(static_cast<const LanePackArgs<PT>*>(onP ? G.dPkP : G.dPkR), r.map, r.blocks,
+                                             G.packWarps, G.packSmem, dim, b, st);
             return;
         }
         {
@@ -1058,7 +1192,8 @@ template <class PT>
 void runChunk(dxg_batch* B, GroupState& G, int n, int dim, int b)
 {
     const int launchesPerIt =
-        5 + (B->amg ? (int)(G.amgP.size() + G.amgR.size()) : (B->redBlack ? 4 : 4 * (int)G.classes.size()));
+        5 + (B->amg ? (int)(G.amgP.size() + G.amgR.size())
+                    : (B->redBlack ? 4 : (G.packs ? 2 * (int)G.rounds.size() : 4 * (int)G.classes.size())));
     cudaStream_t st = B->stream;
     if (B->graphs && !B->timing && !G.exec && !G.graphTried) {
         G.graphTried = true;
@@ -1323,6 +1458,10 @@ void beginIterations(dxg_batch* B, const GroupState& G, const Members& S, const 
         if (fq.empty()) continue;
         launchWaveFactorBatch<PT>(G.classes[q].plan, B->arena.put(fq, st), (int)fq.size(), dim, b, st);
         B->launches += 1;
+    }
+    for (Slot* s : A) {
+        s->packed = false;
+        if (G.packs) packFactor<PT>(B, s);
     }
     std::vector<int64_t> lenM;
     for (Slot* s : A) lenM.push_back(s->c->M);
@@ -1637,6 +1776,13 @@ int dxg_batch_set_memory_budget(dxg_batch* b, int64_t bytes)
 {
     if (!b || bytes < 0) return DXG_ERR_ARG;
     b->budget = bytes;
+    // the packed records give way to the problems
+    if (bytes > 0 && b->bytesInUse + b->packBytes > bytes)
+        return guardedB(b, [&] {
+            DXG_CUDA(cudaSetDevice(b->device));
+            dropPacks(b);
+            return DXG_OK;
+        });
     return DXG_OK;
 }
 
@@ -1660,21 +1806,42 @@ int dxg_batch_add(dxg_batch* b, const dxg_problem_desc* d, const double* u0, dou
         b->err = "admission would exceed the device-memory budget";
         return DXG_ERR_BUDGET;
     }
-    auto s = std::make_unique<Slot>();
-    int st = dxg_ctx_create(&s->c, b->device);
-    if (st != DXG_OK) {
-        b->err = dxg_last_error(nullptr);
-        return st;
-    }
+    std::unique_ptr<Slot> s;
+    int st = DXG_OK;
     auto step = [&](int status) {
         if (status != DXG_OK && b->err.empty()) b->err = dxg_last_error(s->c);
         return status;
     };
-    b->err.clear();
-    if ((st = step(dxg_set_precision(s->c, b->precision))) != DXG_OK) return st;
-    if ((st = step(dxg_problem_upload(s->c, d))) != DXG_OK) return st;
-    if ((st = step(dxg_set_solution(s->c, u0))) != DXG_OK) return st;
-    if ((st = step(dxg_set_prev_solution(s->c, u0))) != DXG_OK) return st;
+    auto make = [&]() -> int {
+        s = std::make_unique<Slot>();
+        b->err.clear();
+        const int made = dxg_ctx_create(&s->c, b->device);
+        if (made != DXG_OK) {
+            b->err = dxg_last_error(nullptr);
+            return made;
+        }
+        if ((st = step(dxg_set_precision(s->c, b->precision))) != DXG_OK) return st;
+        if ((st = step(dxg_problem_upload(s->c, d))) != DXG_OK) return st;
+        if ((st = step(dxg_set_solution(s->c, u0))) != DXG_OK) return st;
+        return step(dxg_set_prev_solution(s->c, u0));
+    };
+    // the packed records give way to the problems
+    auto give = [&] {
+        return guardedB(b, [&] {
+            DXG_CUDA(cudaSetDevice(b->device));
+            dropPacks(b);
+            return DXG_OK;
+        });
+    };
+    if (b->budget > 0 && b->bytesInUse + need + b->packBytes > b->budget && (st = give()) != DXG_OK) return st;
+    st = make();
+    if (st == DXG_ERR_OOM && b->packBytes > 0) {
+        s.reset();
+        if ((st = give()) != DXG_OK) return st;
+        b->noPacks = true;
+        st = make();
+    }
+    if (st != DXG_OK) return st;
     if (params) s->p = *params;
     else dxg_newton_default_params(&s->p);
     if (s->p.enable_partial_reassembly) {
@@ -1771,6 +1938,7 @@ int dxg_batch_remove(dxg_batch* b, int64_t id)
     cudaSetDevice(b->device);
     cudaStreamSynchronize(b->stream);
     b->bytesInUse -= it->second->bytes;
+    b->packBytes -= (int64_t)it->second->c->packMem.bytes();
     b->slots.erase(it);
     return DXG_OK;
 }
@@ -1788,10 +1956,11 @@ int dxg_batch_describe(const dxg_batch* b, char* buf, int64_t len)
                " problems=" + std::to_string(G.ids.size()) + ":";
         if (b->redBlack) out += " [red-black ILU(0): two parallel passes per sweep]";
         if (b->amg) out += " [AMG-BiCGSTAB: " + std::to_string(G.amgP.size()) + " batched passes per V-cycle]";
+        if (G.packs) out += " [packed lane sweeps, " + std::to_string(G.rounds.size()) + " launches per apply]";
         for (const SweepClass& sc : G.classes)
             out += " [" + std::to_string(sc.members.size()) + " problems: cluster " + std::to_string(sc.plan.ctas) +
                    " x " + std::to_string(sc.plan.threads) + " threads, prefetch " + std::to_string(sc.plan.pf) +
-                   "]";
+                   (G.packs ? ", factorisation only]" : "]");
         out += graphsNote(G) + "\n";
     }
     std::strncpy(buf, out.c_str(), (size_t)len - 1);

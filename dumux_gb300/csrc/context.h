@@ -149,6 +149,36 @@ struct dxg_ctx {
 };
 
 namespace dxg {
+// Arguments of the packed sweeps of a planned context.
+template <class T>
+inline LanePackArgs<T> packArgs(dxg_ctx* c, const T* A, const T* L, const T* Dinv, const T* rhs, T* v)
+{
+    const LanePackPlan& p = c->packPlan;
+    LanePackArgs<T> a{};
+    a.nx = c->pcHost.nx;
+    a.ny = c->pcHost.ny;
+    a.nz = c->dim == 3 ? c->pcHost.nz : 1;
+    a.N = c->N;
+    a.nyb = p.nyb;
+    a.warps = p.warps;
+    a.steps = p.steps;
+    a.stages = p.stages;
+    a.ctas = p.ctas;
+    a.clusterSize = p.clusterSize;
+    a.Lf = L;
+    a.A = A;
+    a.Dinv = Dinv;
+    a.pack[0] = c->packMem.get();
+    a.pack[1] = a.pack[0] + lanePackBytes(p, 1, sizeof(T));
+    a.handoff = reinterpret_cast<T*>(a.pack[1] + lanePackBytes(p, -1, sizeof(T)));
+    a.rhs = rhs;
+    a.v = v;
+    a.err = c->singular.get() + 1;
+    a.ks = c->ks.get();
+    a.waitNs = c->waitNs ? c->waitNs : 500000000ull;
+    return a;
+}
+
 // The aggregation AMG levels of a context in value type T (level 0: the Jacobian A with
 // the inverted pivots Dinv, the preconditioner input `in` and output `out`); the coarse
 // levels live in the context's AMG allocation, made on first use.

@@ -189,9 +189,17 @@ __global__ void __launch_bounds__(256) lanePackKernel(LanePackArgs<T> a)
 
 // v = (LU)^-1 rhs: z_i = d_i - L_ix z_x - L_iy z_y - L_iz z_z, then
 // y_i = D_i^-1 (z_i - U_ix y_x - U_iy y_y - U_iz y_z).
-template <class T, int B, int DIM>
-__global__ void __launch_bounds__((kLpMaxWarps + 1) * 32) lanePackApply(LanePackArgs<T> a)
+// BATCH: block k works as CTA map[k].y of problem map[k].x (whole clusters per problem).
+template <class T, int B, int DIM, bool BATCH>
+__global__ void __launch_bounds__((kLpMaxWarps + 1) * 32) lanePackApply(LanePackArgs<T> a0, const LanePackArgs<T>* batch,
+                                                                        const uint2* map)
 {
+    uint2 who = make_uint2(0u, blockIdx.x);
+    if constexpr (BATCH) {
+        who = map[blockIdx.x];
+        a0 = batch[who.x];
+    }
+    const LanePackArgs<T>& a = a0;
     constexpr int R = lpRows<T, B>();
     constexpr int NF = LpRec<B, R, 1, DIM>::n, NB = LpRec<B, R, -1, DIM>::n;
     constexpr int TS = (int)sizeof(T);
@@ -208,15 +216,17 @@ __global__ void __launch_bounds__((kLpMaxWarps + 1) * 32) lanePackApply(LanePack
     cg::cluster_group cluster = cg::this_cluster();
     const int nx = a.nx, ny = a.ny, W = a.warps, steps = a.steps, stages = a.stages;
     const LpSmem lay = lpSmem(steps, W, stages, SS, B, R, DIM, TS);
-    const int cta = (int)blockIdx.x;
+    const int cta = (int)who.y;
     const int lane = threadIdx.x & 31;
     // through a shuffle, so that what depends on it is known to be uniform over the warp
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
     const bool working = cta < a.ctas;
-    const bool producer = warp == W;
+    // the last warp fetches the records; a batched launch has more sweeping warps than some of its
+    // problems use
+    const bool producer = warp == (BATCH ? (int)(blockDim.x >> 5) - 1 : W), idle = BATCH && !producer && warp >= W;
     const LpWhere p = lpWhere<B, R>(working ? cta : 0, a.nyb, W, warp, lane);
     const int yb = working ? cta % a.nyb : 0;
-    const bool lineOk = working && !producer && p.y < ny;
+    const bool lineOk = working && !producer && !idle && p.y < ny;
     const int cs = a.clusterSize;
     // neighbouring CTAs: the planes below and above, the tiles before and after in y
     const int zLo = cta - a.nyb, zHi = cta + a.nyb;
@@ -236,7 +246,7 @@ __global__ void __launch_bounds__((kLpMaxWarps + 1) * 32) lanePackApply(LanePack
     const int yRow = (YP + steps) * B, yDir = (W + 1) * yRow;
 
     // the histories: empty where a value will arrive, zero where the lane has no cell
-    if (!producer) {
+    if (!producer && !idle) {
         if (DIM == 3)
             for (int t = 0; t < steps; ++t) {
                 const int x = t - p.j;
@@ -254,7 +264,7 @@ __global__ void __launch_bounds__((kLpMaxWarps + 1) * 32) lanePackApply(LanePack
         for (int k = threadIdx.x; k < 64; k += W * 32) zero[k] = 0;
         if (lane < kLpMaxStages) lpBarInit(lpAddr(&bars[warp][lane]));
         if (lane == 0) consumed[warp] = 0;
-    } else if (lane == 0) {
+    } else if (producer && lane == 0) {
         stopFlag = 0;
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -265,10 +275,10 @@ __global__ void __launch_bounds__((kLpMaxWarps + 1) * 32) lanePackApply(LanePack
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const bool skip = a.ks && a.ks->status != KS_RUNNING;
 
-    if (producer) {
+    if (producer || idle) {
         // barrier 2 of 3 (the turn): nothing of this warp's orders with it
         asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
-        if (lane == 0 && working && !skip) {
+        if (producer && lane == 0 && working && !skip) {
             int issued[kLpMaxWarps];
 #pragma unroll
             for (int w = 0; w < kLpMaxWarps; ++w) issued[w] = 0;
@@ -581,10 +591,18 @@ __global__ void __launch_bounds__((kLpMaxWarps + 1) * 32) lanePackApply(LanePack
 // ---------------------------------------------------------------- host side
 namespace {
 
-template <class T, int B, int DIM>
-cudaError_t lpLaunch(const LanePackPlan& p, const LanePackArgs<T>& a, cudaStream_t st, int* fits)
+// One problem's launch, a batched one (map), or with `fits` the number of its clusters that are
+// resident at once.
+struct LpShape {
+    unsigned grid;
+    int clusterSize, warps;
+    size_t smem;
+};
+template <class T, int B, int DIM, bool BATCH>
+cudaError_t lpLaunch(const LpShape& p, const LanePackArgs<T>& a, const LanePackArgs<T>* batch, const uint2* map,
+                     cudaStream_t st, int* fits)
 {
-    auto kern = lanePackApply<T, B, DIM>;
+    auto kern = lanePackApply<T, B, DIM, BATCH>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLpSmemLimit);
@@ -592,7 +610,7 @@ cudaError_t lpLaunch(const LanePackPlan& p, const LanePackArgs<T>& a, cudaStream
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.grid);
     cfg.blockDim = dim3((p.warps + 1) * 32);
-    cfg.dynamicSmemBytes = lpSmem(p.steps, p.warps, p.stages, lpStageSteps<T, B, DIM>(), B, lpRows<T, B>(), DIM, (int)sizeof(T)).total;
+    cfg.dynamicSmemBytes = p.smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -610,13 +628,27 @@ cudaError_t lpLaunch(const LanePackPlan& p, const LanePackArgs<T>& a, cudaStream
         if (e != cudaSuccess) cudaGetLastError();
         return cudaSuccess;
     }
-    return cudaLaunchKernelEx(&cfg, kern, a);
+    return cudaLaunchKernelEx(&cfg, kern, a, batch, map);
+}
+template <class T, bool BATCH>
+cudaError_t lpDispatch(int dim, int b, const LpShape& s, const LanePackArgs<T>& a, const LanePackArgs<T>* batch,
+                       const uint2* map, cudaStream_t st, int* fits)
+{
+    if (dim == 3)
+        return b == 2 ? lpLaunch<T, 2, 3, BATCH>(s, a, batch, map, st, fits)
+                      : lpLaunch<T, 1, 3, BATCH>(s, a, batch, map, st, fits);
+    return b == 2 ? lpLaunch<T, 2, 2, BATCH>(s, a, batch, map, st, fits)
+                  : lpLaunch<T, 1, 2, BATCH>(s, a, batch, map, st, fits);
 }
 template <class T>
-cudaError_t lpDispatch(const LanePackPlan& p, const LanePackArgs<T>& a, cudaStream_t st, int* fits)
+int lpStepsPerStage(int dim, int b)
 {
-    if (p.dim == 3) return p.b == 2 ? lpLaunch<T, 2, 3>(p, a, st, fits) : lpLaunch<T, 1, 3>(p, a, st, fits);
-    return p.b == 2 ? lpLaunch<T, 2, 2>(p, a, st, fits) : lpLaunch<T, 1, 2>(p, a, st, fits);
+    return dim == 3 ? (b == 2 ? lpStageSteps<T, 2, 3>() : lpStageSteps<T, 1, 3>()) : lpStageSteps<T, 1, 2>();
+}
+template <class T>
+size_t lpSmemOf(const LanePackPlan& p)
+{
+    return lpSmem(p.steps, p.warps, p.stages, lpStepsPerStage<T>(p.dim, p.b), p.b, p.rows, p.dim, (int)sizeof(T)).total;
 }
 }  // namespace
 
@@ -630,8 +662,19 @@ size_t laneHandoffBytes(const LanePackPlan& p, size_t tsize)
     return 2 * (size_t)p.ctas * p.warps * p.steps * 32 * p.rows * tsize;
 }
 
+template <class T, bool BATCH>
+static int lpResident(const LanePackPlan& p, int warps, size_t smem)
+{
+    int n = 0;
+    lpDispatch<T, BATCH>(p.dim, p.b, LpShape{(unsigned)p.grid, p.clusterSize, warps, smem}, LanePackArgs<T>{}, nullptr,
+                         nullptr, 0, &n);
+    return n;
+}
+
+// whole: clusters of exactly maxCluster CTAs, and where possible little enough shared memory for
+// two CTAs on an SM (a batched launch: its problems share one cluster size and the SMs)
 template <class T>
-static LanePackPlan lpPlanFor(int dim, int nx, int ny, int nz, int b, int warps, int maxCluster)
+static LanePackPlan lpPlanFor(int dim, int nx, int ny, int nz, int b, int warps, int maxCluster, bool whole = false)
 {
     LanePackPlan p{};
     p.dim = dim;
@@ -643,24 +686,25 @@ static LanePackPlan lpPlanFor(int dim, int nx, int ny, int nz, int b, int warps,
     const int tile = warps * lpw;
     p.nyb = (ny + tile - 1) / tile;
     const int64_t ctas = (int64_t)p.nyb * (dim == 3 ? nz : 1);
-    if (p.nyb > maxCluster || ctas > 4096) return p;
+    if (p.nyb > maxCluster || (whole && maxCluster % p.nyb != 0) || ctas > 4096) return p;
     // whole planes, split evenly over as few clusters as hold them
     const int planes = (int)ctas / p.nyb, most = maxCluster / p.nyb;
     const int clusters = (planes + most - 1) / most;
-    const int clusterSize = (planes + clusters - 1) / clusters * p.nyb;
+    const int clusterSize = whole ? maxCluster : (planes + clusters - 1) / clusters * p.nyb;
     // the deepest record ring that fits, at least two stages
-    p.stages = kLpMaxStages;
-    const int stageSteps = dim == 3 ? (b == 2 ? lpStageSteps<T, 2, 3>() : lpStageSteps<T, 1, 3>()) : lpStageSteps<T, 1, 2>();
-    auto smem = [&] { return lpSmem(p.steps, warps, p.stages, stageSteps, b, p.rows, dim, (int)sizeof(T)).total; };
-    while (p.stages > 1 && smem() > kLpSmemLimit) --p.stages;
-    if (p.stages < 2) return p;
+    auto deepest = [&](size_t limit) {
+        p.stages = kLpMaxStages;
+        while (p.stages > 1 && lpSmemOf<T>(p) > limit) --p.stages;
+        return p.stages >= 2;
+    };
+    if (!(whole && deepest(112 * 1024)) && !deepest(kLpSmemLimit)) return p;
     p.ctas = (int)ctas;
     p.clusterSize = clusterSize;
     p.grid = (p.ctas + clusterSize - 1) / clusterSize * clusterSize;
     // every cluster of the launch resident at once
-    int fit = 0;
-    lpDispatch<T>(p, LanePackArgs<T>{}, 0, &fit);
-    p.ok = fit >= p.grid / clusterSize;
+    const int resident = whole ? lpResident<T, true>(p, p.warps, lpSmemOf<T>(p))
+                               : lpResident<T, false>(p, p.warps, lpSmemOf<T>(p));
+    p.ok = resident >= p.grid / clusterSize;
     return p;
 }
 
@@ -685,6 +729,37 @@ LanePackPlan makeLanePackPlan(int dim, int nx, int ny, int nz, int b)
         }
     return LanePackPlan{};
 }
+template <class T>
+LanePackPlan makeLanePackBatchPlan(int dim, int nx, int ny, int nz, int b)
+{
+    if ((dim != 2 && dim != 3) || (b != 1 && b != 2) || nx < 1 || ny < 1 || nz < 1) return LanePackPlan{};
+    const int lpw = 32 * (b == 2 ? lpRows<T, 2>() : 1) / b;
+    auto perPlane = [&](int w) { return (ny + w * lpw - 1) / (w * lpw); };
+    int order[3] = {1, 2, 3};
+    std::stable_sort(order, order + 3, [&](int p, int q) { return perPlane(p) < perPlane(q); });
+    for (int w : order) {
+        const LanePackPlan p = lpPlanFor<T>(dim, nx, ny, nz, b, w, kLanePackBatchCluster, true);
+        if (p.ok) return p;
+    }
+    return LanePackPlan{};
+}
+template <class T>
+int lanePackResident(const LanePackPlan& p, int warps, size_t smem)
+{
+    return lpResident<T, true>(p, warps, smem);
+}
+template <class T>
+size_t lanePackSmem(const LanePackPlan& p)
+{
+    return lpSmemOf<T>(p);
+}
+template <class T>
+void launchLanePackApplyBatch(const LanePackArgs<T>* batch, const uint2* map, unsigned blocks, int warps, size_t smem,
+                              int dim, int b, cudaStream_t st)
+{
+    const LpShape shape{blocks, kLanePackBatchCluster, warps, smem};
+    DXG_CUDA((lpDispatch<T, true>(dim, b, shape, LanePackArgs<T>{}, batch, map, st, nullptr)));
+}
 
 template <class T>
 void launchLanePack(const LanePackPlan& p, const LanePackArgs<T>& a, cudaStream_t st)
@@ -703,11 +778,22 @@ void launchLanePack(const LanePackPlan& p, const LanePackArgs<T>& a, cudaStream_
 template <class T>
 void launchLanePackApply(const LanePackPlan& p, const LanePackArgs<T>& a, cudaStream_t st)
 {
-    DXG_CUDA(lpDispatch<T>(p, a, st, nullptr));
+    const LpShape shape{(unsigned)p.grid, p.clusterSize, p.warps, lpSmemOf<T>(p)};
+    DXG_CUDA((lpDispatch<T, false>(p.dim, p.b, shape, a, nullptr, nullptr, st, nullptr)));
 }
 
 template LanePackPlan makeLanePackPlan<double>(int, int, int, int, int);
+template LanePackPlan makeLanePackBatchPlan<double>(int, int, int, int, int);
+template size_t lanePackSmem<double>(const LanePackPlan&);
+template int lanePackResident<double>(const LanePackPlan&, int, size_t);
+template void launchLanePackApplyBatch<double>(const LanePackArgs<double>*, const uint2*, unsigned, int, size_t, int, int,
+                                           cudaStream_t);
 template LanePackPlan makeLanePackPlan<float>(int, int, int, int, int);
+template LanePackPlan makeLanePackBatchPlan<float>(int, int, int, int, int);
+template size_t lanePackSmem<float>(const LanePackPlan&);
+template int lanePackResident<float>(const LanePackPlan&, int, size_t);
+template void launchLanePackApplyBatch<float>(const LanePackArgs<float>*, const uint2*, unsigned, int, size_t, int, int,
+                                           cudaStream_t);
 template void launchLanePack<double>(const LanePackPlan&, const LanePackArgs<double>&, cudaStream_t);
 template void launchLanePack<float>(const LanePackPlan&, const LanePackArgs<float>&, cudaStream_t);
 template void launchLanePackApply<double>(const LanePackPlan&, const LanePackArgs<double>&, cudaStream_t);

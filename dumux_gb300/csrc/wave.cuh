@@ -87,6 +87,21 @@ struct LanePackPlan {
 // The plan of a grid (ok: shared memory holds the histories and every cluster is resident).
 template <class T>
 LanePackPlan makeLanePackPlan(int dim, int nx, int ny, int nz, int b);
+// Batched launches: plans whose clusters all have kLanePackBatchCluster CTAs; a launch takes
+// problems whose clusters (of `warps` sweeping warps and `smem` bytes per CTA) are resident
+// together, block k of it working as CTA map[k].y of problem map[k].x.  Sixteen: the hand-off between
+// clusters goes through global memory (an ensemble of twelve grids of 16 to 40 cells a side spends
+// 301 ms in the sweeps, 321 ms with clusters of 8 and 424 ms with clusters of 4).
+constexpr int kLanePackBatchCluster = 16;
+template <class T>
+LanePackPlan makeLanePackBatchPlan(int dim, int nx, int ny, int nz, int b);
+template <class T>
+size_t lanePackSmem(const LanePackPlan& p);
+template <class T>
+int lanePackResident(const LanePackPlan& p, int warps, size_t smem);
+template <class T>
+void launchLanePackApplyBatch(const LanePackArgs<T>* batch, const uint2* map, unsigned blocks, int warps, size_t smem,
+                              int dim, int b, cudaStream_t st);
 size_t lanePackBytes(const LanePackPlan& p, int dir, size_t tsize);
 size_t laneHandoffBytes(const LanePackPlan& p, size_t tsize);
 template <class T>

@@ -3,7 +3,7 @@ same bits) at the edges of their tiles, warps and clusters, and their bounded wa
 import numpy as np
 import pytest
 
-from dumux_gb300 import Context, problems
+from dumux_gb300 import Batch, Context, newton_params, problem_device_bytes, problems
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +92,42 @@ def test_packed_mpfa_sweeps_wait_limit_expires_and_the_context_recovers():
     ctx.set_wait_limit(0.5)
     assert ctx.linear_solve(1e-10, 500)["iterations"] == first["iterations"]
     assert np.array_equal(ctx.update(), x0)
+
+
+# problems of one, two and three clusters of CTAs and of one to three sweeping warps in one launch
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("eqs,grids", [
+    (2, [(16, 31, 3), (5, 33, 17), (17, 9, 33), (2, 1, 1), (6, 97, 4), (30, 16, 16)]),
+    (2, [(12, 17), (40, 50), (3, 100), (9, 1)]),
+    (1, [(9, 33, 5), (6, 70, 18), (20, 8, 40)]),
+])
+def test_batched_packed_sweeps_equal_batched_wavefront(eqs, grids, precision):
+    """A memory budget that leaves no room for the packed records keeps the batch on the cluster
+    wavefront; one that shrinks between iterations moves it there in mid-solve, one that is lifted
+    brings the records back when the membership changes.  The solutions are the same bits."""
+    probs = [problems.darcy_1p(cells=g, seed=k) if eqs == 1 else
+             problems.dnapl_2p(cells=g, extent=(6.0, 4.0, 1.0)[:len(g)], seed=k) for k, g in enumerate(grids)]
+    params = newton_params(linear_max_iter=500)
+
+    def run(budget, changes=()):
+        batch = Batch(precision=precision, memory_budget=budget)
+        dt = 250.0 if eqs == 2 else 0.0
+        ids = [batch.add(d, u0, dt=dt, t_end=2 * dt, params=params) for d, u0 in probs]
+        how, n = [], 0
+        while batch.iterate():
+            how.append("packed" in batch.describe())
+            for at, value in changes:
+                if at == n:
+                    batch.set_memory_budget(value)
+            n += 1
+        return [batch.solution(i) for i in ids], how
+
+    tight = sum(problem_device_bytes(d, precision) for d, _ in probs)
+    waves, how = run(tight)
+    assert not any(how)
+    packed, how = run(0)
+    assert all(how)
+    moved, how = run(0, [(1, tight), (3, 0)])
+    assert not eqs == 2 or not all(how)
+    for a, b, c in zip(waves, packed, moved):
+        assert np.array_equal(a, b) and np.array_equal(a, c)
