@@ -32,6 +32,7 @@ UNITS = {
     "mpfa.cu": ["--fmad=false"],
     "stencilwave.cu": [],
     "stencilpack.cu": [],
+    "stencilplane.cu": [],
     "stencillane.cu": [],
     "linesweep.cu": [],
 }

@@ -597,6 +597,7 @@ void tabulate(dxg_ctx* c, const dxg_problem_desc* d)
     c->laneHandoffBytes = 0;
     c->packPlan = LanePackPlan{};
     c->stencilPack = StencilPackPlan{};
+    c->stencilPlane = StencilPlanePlan{};
     c->packPlanned = false;
     c->packMem.release();
     c->waveTuneCount = 0;
@@ -767,6 +768,7 @@ void tabulateMpfa(dxg_ctx* c, const dxg_problem_desc* d)
     c->laneHandoffBytes = 0;
     c->packPlan = LanePackPlan{};
     c->stencilPack = StencilPackPlan{};
+    c->stencilPlane = StencilPlanePlan{};
     c->packPlanned = false;
     c->packMem.release();
     c->waveTuneCount = 0;
@@ -929,10 +931,11 @@ MpfaArgs mpfaArgs(const dxg_ctx* c)
 }
 
 // The MPFA-O preconditioner apply: 4 the line sweeps over packed records (2D, one unknown: auto
-// wherever their plan fits; 256 x 256: 0.30 ms per apply against 0.667 ms for kind 1), 1 the
-// one-CTA line sweeps (2D with up to 1024 lines:
-// DXG_ILU_WAVEFRONT or auto), 2 the cluster line sweeps (2D: DXG_ILU_LANES, or auto beyond
-// 1024 lines), 3 the 3D cluster sweeps (one z-plane per CTA: DXG_ILU_LANES or auto), 0 the
+// wherever their plan fits; 256 x 256: 0.30 ms per apply against 0.667 ms for kind 1), 5 those of
+// the 3D stencil (auto wherever their plan fits; 32 x 32 x 16 2x2 blocks: 0.20 ms against 0.56 ms
+// for kind 3), 1 the one-CTA line sweeps (2D with up to 1024 lines: DXG_ILU_WAVEFRONT or auto),
+// 2 the cluster line sweeps (2D: DXG_ILU_LANES, or auto beyond 1024 lines), 3 the 3D cluster
+// sweeps (one z-plane per CTA: DXG_ILU_LANES or auto), 0 the
 // level-by-level kernel (DXG_ILU_LEVELS, or when none fits).  On 256 x 256 the one-CTA sweeps
 // took 1.09 ms per apply, the cluster sweeps (two CTAs, polled hand-offs between warps)
 // 1.0-2.4 ms.
@@ -943,7 +946,7 @@ int mpfaSweep(const dxg_ctx* c, const StencilArgs& sa)
     case DXG_ILU_LEVELS: return 0;
     case DXG_ILU_LANES: return lanes ? 2 : lanes3 ? 3 : 0;
     case DXG_ILU_WAVEFRONT: return wave ? 1 : 0;
-    default: return c->stencilPack.ok ? 4 : wave ? 1 : lanes ? 2 : lanes3 ? 3 : 0;
+    default: return c->stencilPack.ok ? 4 : c->stencilPlane.ok ? 5 : wave ? 1 : lanes ? 2 : lanes3 ? 3 : 0;
     }
 }
 
@@ -969,9 +972,10 @@ StencilArgs stencilArgs(dxg_ctx* c)
     std::memcpy(a.tri, c->mpTri, sizeof(a.tri));
     a.err = c->singular.get() + 1;
     a.waitNs = c->waitNs;
-    if (c->packMem.get() && c->stencilPack.ok) {
+    if (c->packMem.get() && (c->stencilPack.ok || c->stencilPlane.ok)) {
         a.pack[0] = c->packMem.get();
-        a.pack[1] = a.pack[0] + stencilPackBytes(c->stencilPack, 1);
+        a.pack[1] = a.pack[0] + (c->stencilPack.ok ? stencilPackBytes(c->stencilPack, 1)
+                                                   : stencilPlaneBytes(a, c->stencilPlane, 1));
     }
     return a;
 }
@@ -1176,20 +1180,26 @@ void preparePack(dxg_ctx* c)
     DXG_CUDA(cudaMemsetAsync(c->packMem.get() + records, 0xff, handoff, c->stream));
 }
 
-// As preparePack, for the scalar 2D MPFA-O stencil.
+// As preparePack, for the MPFA-O stencils (2D scalar, 3D).
 void prepareStencilPack(dxg_ctx* c)
 {
     if (!c->packPlanned) {
         c->packPlanned = true;
         c->stencilPack = makeStencilPackPlan(stencilArgs(c));
+        c->stencilPlane = makeStencilPlanePlan(stencilArgs(c));
     }
-    if (!c->stencilPack.ok || c->packMem.get()) return;
+    if ((!c->stencilPack.ok && !c->stencilPlane.ok) || c->packMem.get()) return;
     try {
-        c->packMem.alloc(stencilPackBytes(c->stencilPack, 1) + stencilPackBytes(c->stencilPack, -1));
+        if (c->stencilPack.ok) {
+            c->packMem.alloc(stencilPackBytes(c->stencilPack, 1) + stencilPackBytes(c->stencilPack, -1));
+        } else {
+            const StencilArgs a = stencilArgs(c);
+            c->packMem.alloc(stencilPlaneBytes(a, c->stencilPlane, 1) + stencilPlaneBytes(a, c->stencilPlane, -1));
+        }
     } catch (const Error& e) {
         if (e.status != DXG_ERR_OOM) throw;
         cudaGetLastError();
-        c->stencilPack.ok = false;
+        c->stencilPack.ok = c->stencilPlane.ok = false;
     }
 }
 
@@ -1432,10 +1442,10 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
                 launchStencilFactor(stencilArgs(c), st);
                 c->launches += 1;
                 prepareStencilPack(c);
-                if (c->stencilPack.ok) {   // whatever kernel is set: it may be changed without a new factor
-                    launchStencilPack(stencilArgs(c), c->stencilPack, st);
-                    c->launches += 1;
-                }
+                // whatever kernel is set: it may be changed without a new factor
+                if (c->stencilPack.ok) launchStencilPack(stencilArgs(c), c->stencilPack, st);
+                else if (c->stencilPlane.ok) launchStencilPlanePack(stencilArgs(c), c->stencilPlane, st);
+                c->launches += c->stencilPack.ok || c->stencilPlane.ok;
             }
         } else if (c->linearSolver == DXG_LINEAR_SOLVER_AMG_BICGSTAB) {
             // AMG setup: fine pivots, then each coarse operator (with its pivots) from the one above
@@ -1506,6 +1516,7 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
             if (c->mpfa) {
                 TimedScope ts(c, DXG_KC_ILU_SWEEP, c->bytesSweep);
                 switch (mpfaSweep(c, sa)) {
+                case 5: launchStencilPlaneApply(sa, c->stencilPlane, in, yOut, st); return 1;
                 case 4: launchStencilPackApply(sa, c->stencilPack, in, yOut, st); return 1;
                 case 3: launchStencilLane3d(sa, in, yOut, st); return 2;
                 case 2: launchStencilLane2d(sa, in, yOut, st); return 2;
@@ -2200,6 +2211,9 @@ int dxg_describe(const dxg_ctx* c, char* buf, int64_t len)
         const int k = mpfaSweep(c, sa);
         out = std::string("MPFA-O, ") + std::to_string(c->mpLayout.S) + "-point stencil; ILU(0): natural order, " +
               (k == 3   ? "line sweeps (one lane per grid line and block row, levels x+2y+4z), one z-plane "
+                          "per CTA over a cluster of " +
+                            std::to_string(sa.nz) + " CTAs"
+               : k == 5 ? "line sweeps over packed records (four warps per tile of lines, levels x+2y+4z), one z-plane "
                           "per CTA over a cluster of " +
                             std::to_string(sa.nz) + " CTAs"
                : k == 2 ? "line sweeps (one thread per grid line, levels x+2y) over a cluster of " +

@@ -122,6 +122,7 @@ struct dxg_ctx {
     // plan fits; planned at the first factorisation that uses them
     dxg::LanePackPlan packPlan;
     dxg::StencilPackPlan stencilPack;     // ... and of the 2D scalar MPFA-O stencil
+    dxg::StencilPlanePlan stencilPlane;   // ... and of the 3D one
     bool packPlanned = false;
     dxg::DevBuf<unsigned char> packMem;   // records of both sweeps, then the hand-off buffer
     dxg::DevBuf<unsigned char> laneHandoff;

@@ -141,7 +141,7 @@ struct StencilArgs {
     int8_t tri[104][3] = {};
     int* err = nullptr;                    // DXG_ERR_TIMEOUT of a sweep that gave up waiting
     unsigned long long waitNs = 0;         // wait limit of the cluster sweeps (0: 0.5 s)
-    unsigned char* pack[2] = {};           // packed records of the forward / backward sweep (stencilpack.cu)
+    unsigned char* pack[2] = {};           // packed records of the forward / backward sweep (stencilpack.cu, stencilplane.cu)
 };
 // Sweeps of the scalar 2D 9-point stencil over packed records (stencilpack.cu), one cluster.
 struct StencilPackPlan {
@@ -152,6 +152,16 @@ StencilPackPlan makeStencilPackPlan(const StencilArgs& a);
 size_t stencilPackBytes(const StencilPackPlan& p, int dir);
 void launchStencilPack(const StencilArgs& a, const StencilPackPlan& p, cudaStream_t st);
 void launchStencilPackApply(const StencilArgs& a, const StencilPackPlan& p, const double* d, double* v, cudaStream_t st);
+// Sweeps of the 3D 27-point stencil over packed records (stencilplane.cu): one z-plane per CTA
+// (nz <= 16), four warps per tile of lines.
+struct StencilPlanePlan {
+    bool ok = false;
+    int tiles = 0, steps = 0, stages = 0;   // tiles per plane, padded steps per tile, ring depth
+};
+StencilPlanePlan makeStencilPlanePlan(const StencilArgs& a);
+size_t stencilPlaneBytes(const StencilArgs& a, const StencilPlanePlan& p, int dir);
+void launchStencilPlanePack(const StencilArgs& a, const StencilPlanePlan& p, cudaStream_t st);
+void launchStencilPlaneApply(const StencilArgs& a, const StencilPlanePlan& p, const double* d, double* v, cudaStream_t st);
 void launchStencilSpmv(const StencilArgs& a, const double* x, double* y, const double* w, int mode, cudaStream_t st);
 void launchStencilFactor(const StencilArgs& a, cudaStream_t st);
 // the preconditioner apply: the level-by-level kernel (any stencil), the one-CTA line sweeps

@@ -131,3 +131,45 @@ def test_batched_packed_sweeps_equal_batched_wavefront(eqs, grids, precision):
     assert not eqs == 2 or not all(how)
     for a, b, c in zip(waves, packed, moved):
         assert np.array_equal(a, b) and np.array_equal(a, c)
+
+
+# tiles of 16 (2x2) or 32 lines, up to four; one to sixteen planes
+@pytest.mark.parametrize("b,cells", [
+    (1, (3, 4, 1)), (1, (5, 32, 3)), (1, (6, 33, 16)), (1, (4, 128, 2)), (1, (40, 9, 5)),
+    (2, (2, 2, 2)), (2, (5, 16, 3)), (2, (8, 17, 16)), (2, (3, 33, 5)), (2, (9, 64, 2)), (2, (40, 7, 6)),
+])
+def test_packed_mpfa_plane_sweeps_equal_level_kernel(b, cells):
+    if b == 1:
+        desc, prev, _ = problems.mpfa_linear_field_problem(
+            cells=cells, K=((2.0, 0.3, 0.1), (0.3, 1.0, 0.2), (0.1, 0.2, 1.5)), spacing_seed=2)
+        u, dt = prev, 0.0
+    else:
+        desc, prev = problems.dnapl_2p_mpfa(cells=cells, seed=6)
+        u = prev.reshape(-1, 2).copy()
+        u[:, 1] = np.random.default_rng(9).uniform(0, 0.4, len(u))
+        u, dt = u.reshape(-1), 250.0
+    n0, x0, _ = _solve(desc, u, prev, "levels", "fp64", dt)
+    n1, x1, how = _solve(desc, u, prev, "auto", "fp64", dt)
+    assert "packed records" in how and "one z-plane per CTA" in how
+    assert n1 == n0
+    assert np.array_equal(x1, x0)
+
+
+def test_packed_mpfa_plane_sweeps_wait_limit_expires_and_the_context_recovers():
+    desc, u0 = problems.dnapl_2p_mpfa(cells=(16, 20, 16), seed=6)
+    u = u0.reshape(-1, 2).copy()
+    u[:, 1] = np.random.default_rng(9).uniform(0, 0.4, len(u))
+    ctx = Context(desc)
+    ctx.set_solution(u.reshape(-1))
+    ctx.set_prev_solution(u0)
+    ctx.set_time_step(250.0)
+    ctx.assemble_jacobian_and_residual()
+    first = ctx.linear_solve(1e-10, 500)
+    assert first["converged"] and "packed records" in ctx.describe()
+    x0 = ctx.update()
+    ctx.set_wait_limit(1e-6)
+    with pytest.raises(Exception, match="timed out"):
+        ctx.linear_solve(1e-10, 500)
+    ctx.set_wait_limit(0.5)
+    assert ctx.linear_solve(1e-10, 500)["iterations"] == first["iterations"]
+    assert np.array_equal(ctx.update(), x0)
