@@ -339,10 +339,15 @@ cudaError_t slLaunch(const StencilArgs& a, const double* d, double* v, cudaStrea
 // stores it) and the update triples (s, t, u) of one s, whose targets t differ, run on separate
 // lanes; a cluster barrier ends each level.  Products, operand order and FMAs are those of
 // stencilFactorKernel / stencilFactor2Kernel, so the factors are the same bits.  Before a row's
-// elimination its warp stages everything the row reads (its blocks, the lower neighbours'
-// pivots, masks and the neighbour blocks of every update triple) in shared memory with all loads
-// in flight together: one memory latency per row instead of one per lower slot.  Rows of
-// earlier levels are read past L1 (ld.global.cg): another SM of the cluster wrote them.
+// elimination its warp stages everything the row reads (its blocks and masks a level ahead, the
+// lower neighbours' pivots and the neighbour blocks of every update triple) in shared memory with
+// all loads in flight together (2x2 blocks: asynchronous copies): one memory latency per row.  Rows
+// of earlier levels are read past L1: another SM of the cluster wrote them.
+//
+// What bounds it: the levels, each a chain of 13 slots (~10 dependent FP64 instructions of 64 cycles
+// with the shuffles and shared-memory round trips between them) and a barrier.  32x32x16 2x2 blocks:
+// 1.7 ms; with the copies through registers in turn and the rows filling one CTA after the other
+// 3.5 ms.
 constexpr int kSfWarps = 16;
 constexpr int kSfCtas = 16;
 
@@ -375,20 +380,41 @@ __host__ __device__ constexpr size_t sfWarpBytes()
     return (size_t)(27 + 13 + 104) * B * B * sizeof(double) + 64;
 }
 
+// A piece of a block into shared memory, past L1 (another SM of the cluster may have written it), or
+// zeros: 16 bytes of a 2x2 block asynchronously, the entry of a 1x1 block through a register.
+template <int BB>
+__device__ __forceinline__ void sfCopy(double* dst, const double* src, bool ok)
+{
+    if constexpr (BB == 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(slSmem(dst)), "l"(src), "r"(ok ? 16 : 0)
+                     : "memory");
+    else
+        *dst = ok ? __ldcg(src) : 0.0;
+}
+
 template <int B>
 __global__ void __launch_bounds__(kSfWarps * 32) stencilFactorClusterKernel(StencilArgs a)
 {
-    constexpr int BB = B * B;
+    constexpr int BB = B * B, CH = BB == 4 ? 2 : 1, PER = BB / CH;   // a block is CH copies of PER entries
     extern __shared__ __align__(16) unsigned char sfRaw[];
     // the update triples in shared memory: lanes read different triples, which from the kernel
     // parameters (constant bank) would serialise
     __shared__ int8_t tri[104][3];
+    __shared__ int first[15];   // the update triples of lower slot s: first[s] .. first[s + 1] - 1
     for (int e = threadIdx.x; e < a.nTri * 3; e += blockDim.x) tri[e / 3][e % 3] = a.tri[e / 3][e % 3];
+    __syncthreads();
+    if (threadIdx.x < 15) {
+        int n = 0;
+        while (n < a.nTri && tri[n][0] < (int)threadIdx.x) ++n;
+        first[threadIdx.x] = n;
+    }
     __syncthreads();
     cg::cluster_group cluster = cg::this_cluster();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nW = (int)gridDim.x * kSfWarps;
-    const int gw = (int)blockIdx.x * kSfWarps + warp;
+    // a level's rows go round the CTAs first: a row takes ~100 FP64 instructions of 64 cycles on its
+    // warp's sub-partition, so few rows per sub-partition are what a level's time is made of
+    const int gw = warp * (int)gridDim.x + (int)blockIdx.x;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
     const int64_t N = a.N;
     const int S = a.S, center = a.center, nTri = a.nTri;
@@ -397,55 +423,66 @@ __global__ void __launch_bounds__(kSfWarps * 32) stencilFactorClusterKernel(Sten
     double* Dn = R + 27 * BB;
     double* Un = Dn + 13 * BB;
     uint32_t* Mn = reinterpret_cast<uint32_t*>(Un + 104 * BB);
+    // what a row needs from the matrix alone, also a level ahead: its mask, its blocks and the masks
+    // of its lower neighbours
+    uint32_t m = 0;
+    auto stageOwn = [&](int64_t i) {
+        m = __ldg(a.mask + i);
+        for (int e = lane; e < S * CH; e += 32)
+            sfCopy<BB>(R + e * PER, a.A + ((int64_t)(e / CH) * N + i) * BB + e % CH * PER, true);
+        for (int s = lane; s < center; s += 32) Mn[s] = ((m >> s) & 1u) ? __ldg(a.mask + i + a.off[s]) : 0u;
+    };
+    int64_t i;
+    bool ahead = sfLevelRow(0, gw, nx, ny, nz, i);
+    if (ahead) stageOwn(i);
     for (int L = 0; L < levels; ++L) {
-        int64_t i;
         for (int k = gw; sfLevelRow(L, k, nx, ny, nz, i); k += nW) {
-            const uint32_t m = __ldg(a.mask + i);
-            // everything the row reads, staged with all loads in flight together
-            for (int e = lane; e < S * BB; e += 32) R[e] = a.A[((int64_t)(e / BB) * N + i) * BB + e % BB];
-            for (int e = lane; e < center * BB; e += 32) {
-                const int s = e / BB;
-                Dn[e] = ((m >> s) & 1u) ? __ldcg(a.Dinv + (i + a.off[s]) * BB + e % BB) : 0.0;
+            if (!ahead) stageOwn(i);
+            ahead = false;
+            // the lower neighbours' pivots and their blocks, all loads in flight together
+            for (int e = lane; e < center * CH; e += 32) {
+                const int s = e / CH;
+                const bool ok = (m >> s) & 1u;
+                sfCopy<BB>(Dn + e * PER, a.Dinv + (i + (ok ? a.off[s] : 0)) * BB + e % CH * PER, ok);
             }
-            for (int s = lane; s < center; s += 32) Mn[s] = ((m >> s) & 1u) ? __ldg(a.mask + i + a.off[s]) : 0u;
-            for (int e = lane; e < nTri * BB; e += 32) {
-                const int kk = e / BB;
+#pragma unroll 4
+            for (int e = lane; e < nTri * CH; e += 32) {
+                const int kk = e / CH;
                 const int s = tri[kk][0], t = tri[kk][1], u = tri[kk][2];
-                Un[e] = (((m >> s) & 1u) && ((m >> t) & 1u))
-                            ? __ldcg(a.LU + ((int64_t)u * N + i + a.off[s]) * BB + e % BB)
-                            : 0.0;
+                const bool ok = ((m >> s) & 1u) && ((m >> t) & 1u);
+                sfCopy<BB>(Un + e * PER, a.LU + ((int64_t)u * N + i + (ok ? a.off[s] : 0)) * BB + e % CH * PER, ok);
             }
+            asm volatile("cp.async.wait_all;" ::: "memory");
             __syncwarp();
-            int t0 = 0;
             // 2x2 blocks: lane q works on entry e = q % 4 (row er, column ec) of update triple
             // t0 + q / 4 + 8 n; every entry of a block product is its own two-FMA chain, so this
-            // is the arithmetic of the whole-block products with 3 FP64 instructions per lane and
+            // is the arithmetic of the whole-block products with 5 FP64 instructions per lane and
             // lower slot instead of 12 per triple
             const int e4 = lane & 3, er = e4 >> 1, ec = e4 & 1;
             for (int s = 0; s < center; ++s) {
                 if (!((m >> s) & 1u)) continue;
                 const uint32_t mj = Mn[s];
-                while (t0 < nTri && tri[t0][0] < s) ++t0;
+                const int t0 = first[s], t1 = first[s + 1];
                 if constexpr (B == 1) {
                     const double l = R[s] * Dn[s];
                     __syncwarp();
                     if (lane == 0) R[s] = l;
-                    for (int k2 = t0 + lane; k2 < nTri && tri[k2][0] == s; k2 += 32) {
+                    for (int k2 = t0 + lane; k2 < t1; k2 += 32) {
                         const int t = tri[k2][1], u = tri[k2][2];
                         if (((m >> t) & 1u) && ((mj >> u) & 1u)) R[t] = fma(-l, Un[k2], R[t]);
                     }
                 } else {
-                    // row er of the multiplier l = a_is Dinv_j (the entries this lane needs)
+                    // entry e4 of the multiplier l = a_is Dinv_j on every lane, its row er by shuffles
                     const double* X = R + s * 4;
                     const double* Y = Dn + s * 4;
-                    double l0 = 0.0, l1 = 0.0;
-                    l0 = fma(X[er * 2 + 0], Y[0 * 2 + 0], l0);
-                    l0 = fma(X[er * 2 + 1], Y[1 * 2 + 0], l0);
-                    l1 = fma(X[er * 2 + 0], Y[0 * 2 + 1], l1);
-                    l1 = fma(X[er * 2 + 1], Y[1 * 2 + 1], l1);
+                    double l = 0.0;
+                    l = fma(X[er * 2 + 0], Y[0 * 2 + ec], l);
+                    l = fma(X[er * 2 + 1], Y[1 * 2 + ec], l);
+                    const double l0 = __shfl_sync(0xffffffffu, l, lane & ~1);
+                    const double l1 = __shfl_sync(0xffffffffu, l, lane | 1);
                     __syncwarp();
-                    if (lane < 4) R[s * 4 + e4] = ec == 0 ? l0 : l1;
-                    for (int k2 = t0 + (lane >> 2); k2 < nTri && tri[k2][0] == s; k2 += 8) {
+                    if (lane < 4) R[s * 4 + e4] = l;
+                    for (int k2 = t0 + (lane >> 2); k2 < t1; k2 += 8) {
                         const int t = tri[k2][1], u = tri[k2][2];
                         if (((m >> t) & 1u) && ((mj >> u) & 1u)) {
                             const double* U = Un + k2 * 4;
@@ -477,6 +514,8 @@ __global__ void __launch_bounds__(kSfWarps * 32) stencilFactorClusterKernel(Sten
             }
             __syncwarp();
         }
+        ahead = L + 1 < levels && sfLevelRow(L + 1, gw, nx, ny, nz, i);
+        if (ahead) stageOwn(i);
         cluster.sync();
     }
 }

@@ -189,6 +189,32 @@ def test_mpfa_3d_linear_solve_matches_oracle(b, cells):
     assert abs(res["iterations"] - ores.iterations) <= max(2, 0.1 * ores.iterations)
 
 
+@pytest.mark.parametrize("b", [1, 2])
+def test_mpfa_3d_factor_of_levels_beyond_the_clusters_warps_matches_oracle(b):
+    """Levels of up to 400 rows: some of the 256 warps of the factorisation take a second row, which
+    is not staged a level ahead."""
+    cells = (64, 40, 20)
+    if b == 1:
+        K = ((2.0, 0.3, 0.1), (0.3, 1.0, 0.2), (0.1, 0.2, 1.5))
+        desc, u0, _ = problems.mpfa_linear_field_problem(cells=cells, K=K, spacing_seed=2)
+    else:
+        desc, u0 = problems.dnapl_2p_mpfa(cells=cells, seed=6)
+    ctx = Context(desc)
+    ctx.set_solution(u0)
+    ctx.set_prev_solution(u0)
+    if b == 2:
+        ctx.set_time_step(250.0)
+    ctx.assemble_jacobian_and_residual()
+    res = ctx.linear_solve(1e-13, 1000)
+    assert res["converged"]
+    x = ctx.update()
+    row_ptr, col, vals = ctx.jacobian()
+    st, xo, ores = oracle.linear_solve(row_ptr, col, vals, ctx.residual(), b, reduction=1e-13, max_iter=1000)
+    assert st == 0
+    assert np.max(np.abs(x - xo)) <= 1e-8 * np.max(np.abs(xo))
+    assert abs(res["iterations"] - ores.iterations) <= max(2, 0.1 * ores.iterations)
+
+
 def test_mpfa_3d_cluster_sweep_wait_limit_expires_and_recovers():
     """The 3D cluster sweeps under a 1 us wait limit give up (each plane waits for the plane
     before far longer), the solve reports DXG_ERR_TIMEOUT, and with the limit restored the same
