@@ -70,8 +70,7 @@ def parse():
                     help="Jacobian by numeric differentiation (default, the reference's default) or analytic")
     ap.add_argument("--ilu", default="natural", choices=["natural", "lanes", "wavefront", "redblack"],
                     help="ILU(0) of the single-problem workloads: natural order (the reference's SeqILU, "
-                         "default; the context times the lane sweeps and the cluster wavefront and keeps "
-                         "the faster), natural order forced onto the lane sweeps or onto the cluster "
+                         "default; lane sweeps over packed records where they fit), natural order forced onto the lane sweeps or onto the cluster "
                          "wavefront, or red-black (two parallel passes per sweep, more iterations)")
     ap.add_argument("--solver", default="ilu", choices=["ilu", "amg"],
                     help="ILU(0)-BiCGSTAB (default, the reference's ILUBiCGSTABIstlSolver) or "
@@ -223,10 +222,11 @@ def measured_peaks():
 
 # dram__bytes_read.sum + dram__bytes_write.sum per ILU(0) apply (forward + backward sweep)
 # of the 64x64x32 FP64 system, from ncu captures of the sweeps (cold-cache, serialised
-# launches): the cluster wavefront kernels and the lane sweeps (register-ring form, the one
-# the context picks at this size).
+# launches): the cluster wavefront kernels, the lane sweeps that read the factor in place
+# (register-ring form) and the packed lane sweeps (one launch, the default).
 ILU_TRAFFIC_PER_APPLY_64x64x32 = 14537472 + 18714112
 LANE_TRAFFIC_PER_APPLY_64x64x32 = 14520320 + 18721792
+PACKED_TRAFFIC_PER_APPLY_64x64x32 = 38970368 + 1024
 # DRAM bytes per cell of one batched FP32 apply (forward + backward sweep), from an ncu capture
 # of a 32-problem ensemble (2,379,154 cells); traffic scales with the cells swept (each block
 # and vector entry is moved once)
@@ -605,7 +605,9 @@ def batch_roofline(batch):
                          "algorithmic_bytes_per_launch": (by / n) if n else None}
     top = max(kernels, key=lambda k: kernels[k]["ms"])
     total = sum(v["ms"] for v in kernels.values())
-    names = {"ilu_sweep": "waveKernel (batched ILU(0) forward+backward sweeps, one cluster per problem)",
+    packed = "packed lane sweeps" in batch.describe()
+    names = {"ilu_sweep": "lanePackApply (batched ILU(0) forward+backward lane sweeps)" if packed else
+                          "waveKernel (batched ILU(0) forward+backward sweeps, one cluster per problem)",
              "assembly": "volvarsKernel + rowKernel (batched numeric-diff assembly)",
              "spmv": "spmvKernel (batched block SpMV)"}
     a = kernels[top]["gbs"]
@@ -655,7 +657,7 @@ def run_ensemble(args):
     batch = dumux_gb300.Batch(device=local, precision=args.precision, ilu=args.ilu, solver=args.solver)
     ids = [batch.add(d, u0, dt=dt, t_end=t_end, params=params) for d, u0, _ in probs]
     cells_of = {pid: d.num_cells for pid, (d, _, _) in zip(ids, probs)}
-    ticks(batch, args.warmup * T)            # includes the sweep autotuning
+    ticks(batch, args.warmup * T)            # includes kernel loading
     # kernel-class timing over one step's ticks (events around the batched launches)
     batch.set_kernel_timing(True)
     ticks(batch, T)
@@ -775,7 +777,7 @@ def run_serve(args):
     budget = int(0.8 * free)
     server = Server(device=local, precision=args.precision, memory_budget=budget, params=params, ilu=args.ilu,
                     solver=args.solver)
-    # warm-up: small requests of both kinds (kernel loading, sweep autotuning)
+    # warm-up: small requests of both kinds (kernel loading)
     warm = problems.served_requests(max(3, args.warmup), rate=1e6, seed=99, n_max=2e4)
     server.serve(warm, problems.make_request_problem)
     launches0 = server.batch.kernel_launches()
@@ -1087,7 +1089,9 @@ def main():
     peak, peak_kind = measured_peaks()
     achieved = (sweep_bytes / sweep_n) / (sweep_ms / sweep_n / 1e3) / 1e9 if sweep_n else None
     lanes = "lane wavefront" in ctx.describe().split(";")[0]
-    traffic = ((LANE_TRAFFIC_PER_APPLY_64x64x32 if lanes else ILU_TRAFFIC_PER_APPLY_64x64x32)
+    packed = "packed records" in ctx.describe().split(";")[0]
+    traffic = ((PACKED_TRAFFIC_PER_APPLY_64x64x32 if lanes and packed else
+                LANE_TRAFFIC_PER_APPLY_64x64x32 if lanes else ILU_TRAFFIC_PER_APPLY_64x64x32)
                if (args.workload == "2p" and cells == (64, 64, 32) and args.precision == "fp64") else None)
     if args.solver == "amg":
         rkernel = "AMG V-cycle (amg.cu passes, one preconditioner application)"
@@ -1098,7 +1102,8 @@ def main():
         rnote = "bandwidth-bound passes, latency bound at small grids"
     elif args.workload in ("mpfa", "mpfa2p"):
         dsc = ctx.describe()
-        kname = ("stencilLane3dKernel" if "one z-plane per CTA" in dsc else
+        kname = (("stencilPlaneApply" if "one z-plane per CTA" in dsc else "stencilPackApply") if packed else
+                 "stencilLane3dKernel" if "one z-plane per CTA" in dsc else
                  "stencilLane2dKernel" if "over a cluster" in dsc else
                  "stencilWave2dKernel" if "line sweeps" in dsc else "stencilApplyKernel")
         rkernel = f"{kname} (ILU(0) forward+backward sweep of the MPFA-O stencil, one apply)"
@@ -1106,7 +1111,8 @@ def main():
                  "algorithmic bytes: every factor entry, pivot and vector entry once")
         traffic = None
     elif lanes:
-        rkernel = "laneWaveKernel (ILU(0) forward+backward lane sweeps, one apply)"
+        rkernel = (("lanePackApply" if packed else "laneWaveKernel") +
+                   " (ILU(0) forward+backward lane sweeps, one apply)")
         rnote = ("latency/FP64-bound wavefront (one dependent level per grid line step and plane), "
                  "far below the HBM roof")
     else:

@@ -254,14 +254,15 @@ class Context:
         return self._L.dxg_suggest_time_step(self._h, float(old_dt), C.byref(p))
 
     def set_lane_ring(self, form):
-        """Form of the lane sweeps: 'auto' (timed at the first factorisation), 'registers' or
-        'ring' (shared-memory prefetch ring); both give the same bits."""
+        """Form of the lane sweeps: 'auto' (packed factor records where they fit), 'registers' or
+        'ring' (the factor read in place, through registers or a shared-memory ring); all give the
+        same bits."""
         self._check(self._L.dxg_set_lane_ring(self._h, {"auto": 0, "registers": 1, "ring": 2}[form]))
 
     def set_ilu_kernel(self, kind):
-        """'auto' / 'wavefront' (one cluster launch per sweep), 'lanes' (two lanes per grid line,
-        one plane per CTA over several clusters; 3D 2x2 blocks) or 'levels' (one launch per
-        level): the natural-order ILU(0) of the reference; 'redblack': ILU(0) of the red-black
+        """'auto' (lane sweeps over packed records where they fit, else the fastest), 'wavefront'
+        (one cluster launch per sweep), 'lanes' (one lane per grid line and block row, tiles of a
+        plane per CTA over several clusters) or 'levels' (one launch per level): the natural-order ILU(0) of the reference; 'redblack': ILU(0) of the red-black
         reordered matrix (a different preconditioner, two parallel passes per sweep)."""
         self._check(self._L.dxg_set_ilu_kernel(self._h, {"auto": 0, "wavefront": 1, "levels": 2,
                                                           "redblack": 3, "lanes": 4}[kind]))

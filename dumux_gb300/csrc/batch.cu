@@ -868,11 +868,39 @@ void dropPacks(dxg_batch* B)
     B->packBytes = 0;
 }
 
-// Whether a group's natural-order sweeps run over packed records: every member's plan fits, and
-// device memory (or the batch's budget) holds the records beside the problems.  Their buffers are
-// made here.  One launch of the packed sweeps does both directions of several problems: an ensemble
-// of twelve grids of 16 to 40 cells a side takes 0.45 s in FP32 against 0.68 s on the cluster
-// wavefront (six in FP64 0.44 against 0.94 s), twelve of 16 to 22 cells 0.11 against 0.15 s.
+// Which members share a launch: first fit over the members by falling length of their sweeps.
+template <class PT>
+std::vector<std::vector<uint2>> packRounds(const Members& S, int warps, size_t smem)
+{
+    const int room = lanePackResident<PT>(S[0]->c->packPlan, warps, smem) * kLanePackBatchCluster;
+    std::vector<int> order(S.size());
+    for (size_t k = 0; k < S.size(); ++k) order[k] = (int)k;
+    auto length = [&](int k) { return S[k]->c->packPlan.steps + (S[k]->c->dim == 3 ? S[k]->c->pcHost.nz : 0); };
+    std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return length(p) > length(q); });
+    std::vector<std::vector<uint2>> rounds;
+    for (int k : order) {
+        const int grid = S[k]->c->packPlan.grid;
+        size_t r = 0;
+        while (r < rounds.size() && (int)rounds[r].size() + grid > room) ++r;
+        if (r == rounds.size()) rounds.emplace_back();
+        for (int j = 0; j < grid; ++j) rounds[r].push_back(make_uint2((unsigned)k, (unsigned)j));
+    }
+    return rounds;
+}
+
+// Whether a group's natural-order sweeps run over packed records: every member's plan fits, few
+// launches take all members, and device memory (or the batch's budget) holds the records beside the
+// problems.  Their buffers are made here.
+// A launch of the packed sweeps takes about a third of an apply of the cluster wavefront in FP32 and a
+// quarter in FP64, whatever it holds; the wavefront, with its small clusters, holds many problems at
+// once.  Per apply, packed against wavefront: FP32, grids of 16 to 40 cells a side, 12 problems (3
+// launches) 147 against 150 us, 24 (9) 436 against 163, 48 (17) 1024 against 201; 64 grids of 8 to 16
+// (5) 102 against 64; FP64, 24 of 16 to 40 (9) 668 against 305.
+template <class PT>
+constexpr size_t packLaunches()
+{
+    return sizeof(PT) == 8 ? 3 : 2;
+}
 template <class PT>
 bool preparePacks(dxg_batch* B, const Members& S)
 {
@@ -897,6 +925,7 @@ bool preparePacks(dxg_batch* B, const Members& S)
     const int resident = lanePackResident<PT>(S[0]->c->packPlan, warps, smem);
     for (Slot* s : S)
         if (s->c->packPlan.grid / kLanePackBatchCluster > resident) return false;
+    if (packRounds<PT>(S, warps, smem).size() > packLaunches<PT>()) return false;
     if (B->budget > 0 && B->bytesInUse + B->packBytes + need > B->budget) return false;
     for (Slot* s : S) {
         dxg_ctx* c = s->c;
@@ -925,26 +954,6 @@ void packFactor(dxg_batch* B, Slot* s)
     B->launches += 1;
     s->packed = true;
 }
-// Which members share a launch: first fit over the members by falling length of their sweeps.
-template <class PT>
-std::vector<std::vector<uint2>> packRounds(const Members& S, int warps, size_t smem)
-{
-    const int room = lanePackResident<PT>(S[0]->c->packPlan, warps, smem) * kLanePackBatchCluster;
-    std::vector<int> order(S.size());
-    for (size_t k = 0; k < S.size(); ++k) order[k] = (int)k;
-    auto length = [&](int k) { return S[k]->c->packPlan.steps + (S[k]->c->dim == 3 ? S[k]->c->pcHost.nz : 0); };
-    std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return length(p) > length(q); });
-    std::vector<std::vector<uint2>> rounds;
-    for (int k : order) {
-        const int grid = S[k]->c->packPlan.grid;
-        size_t r = 0;
-        while (r < rounds.size() && (int)rounds[r].size() + grid > room) ++r;
-        if (r == rounds.size()) rounds.emplace_back();
-        for (int j = 0; j < grid; ++j) rounds[r].push_back(make_uint2((unsigned)k, (unsigned)j));
-    }
-    return rounds;
-}
-
 // (Re)builds the group's chunk arguments when its membership changed.
 template <class PT>
 GroupState& groupState(dxg_batch* B, const GroupKey& key, const Members& S)

@@ -31,6 +31,11 @@
 //     consumer that starts once its producer is that far ahead.
 // A plane starts its backward sweep as soon as its forward sweep is done (one cluster barrier:
 // the z history is used in both directions), so the turn costs no launch.
+// So a cluster waits for clusters of lower and of higher index, and a launch whose clusters are not
+// all resident would wait for itself: the plan counts them (cudaOccupancyMaxActiveClusters), a
+// batched launch takes no more problems than fit.  Launches of other streams only delay: a grid's
+// CTAs are dispatched whole before those of the next one (sixteen contexts solving on sixteen
+// threads ran without an expired wait).
 // Every history starts filled with an all-ones pattern (a NaN that no arithmetic produces)
 // which the consumer waits to see replaced: each entry is one aligned 4- or 8-byte relaxed
 // store, seen whole, so no fence, flag or barrier sits on the chain.  The consumer puts the

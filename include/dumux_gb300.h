@@ -252,9 +252,11 @@ double dxg_suggest_time_step(const dxg_ctx* ctx, double old_dt, const dxg_newton
 int dxg_advance_time_step(dxg_ctx* ctx);
 
 /* ---- tuning --------------------------------------------------------------------------- */
-/* Kernels of the ILU(0) factorisation and sweeps.  DXG_ILU_AUTO / DXG_ILU_WAVEFRONT: one
- * thread-block-cluster wavefront launch per sweep; DXG_ILU_LEVELS: one launch per
- * wavefront level.  Both compute SeqILU's natural-order ILU(0) (the drop-in setting).
+/* Kernels of the ILU(0) factorisation and sweeps.  DXG_ILU_AUTO: the lane sweeps over packed
+ * factor records where they fit the grid, else the fastest of the other kernels, timed at the
+ * first factorisation; DXG_ILU_WAVEFRONT: one thread-block-cluster wavefront launch per sweep;
+ * DXG_ILU_LEVELS: one launch per wavefront level.  All compute SeqILU's natural-order ILU(0) (the
+ * drop-in setting) with the same bits.
  * DXG_ILU_REDBLACK: ILU(0) of the red-black reordered matrix (cells coloured by the parity
  * of x+y+z) -- a different preconditioner, not the reference's: BiCGSTAB needs more
  * iterations (about 1.6-2.2x on the 2p problems), but a sweep pair is two fully
@@ -262,16 +264,18 @@ int dxg_advance_time_step(dxg_ctx* ctx);
  * same to the linear and Newton tolerances.  No counterpart in the reference (dune-istl's
  * SeqILU is sequential, natural order). */
 enum { DXG_ILU_AUTO = 0, DXG_ILU_WAVEFRONT = 1, DXG_ILU_LEVELS = 2, DXG_ILU_REDBLACK = 3, DXG_ILU_LANES = 4 };
-/* DXG_ILU_LANES: the natural-order sweeps of 3D 2x2-block systems with two lanes per grid line
- * and one z-plane per CTA over several thread-block clusters (more SMs on the level chain);
- * the same factors and arithmetic per cell as DXG_ILU_WAVEFRONT, so the same results.
- * DXG_ILU_AUTO takes it when the timing at the first factorisation finds it faster. */
+/* DXG_ILU_LANES: the natural-order sweeps with one lane per grid line and block row, tiles of a
+ * z-plane per CTA over several thread-block clusters (more SMs on the level chain); the same
+ * factors and arithmetic per cell as DXG_ILU_WAVEFRONT, so the same results.  The factor is
+ * re-laid for them after each factorisation, which takes about its size in device memory more;
+ * where that is not there, the sweeps read the factor in place. */
 int dxg_set_ilu_kernel(dxg_ctx* ctx, int kind);
-/* Form of the lane sweeps: 0 (default) times both at the first factorisation and keeps the
- * faster, 1 the register form (each step's records in a register ring, no vote per step), 2 the
- * shared-memory-ring form (records copied ahead with cp.async, faster where most plane
- * hand-offs cross thread-block clusters); both give the same bits.  DXG_ERR_ARG for 2 when it
- * does not fit the grid.  No counterpart in the reference. */
+/* Form of the lane sweeps: 0 (default) the packed records where they fit, else the faster of the
+ * two forms that read the factor in place, timed at the first factorisation; 1 the register form
+ * (each step's records in a register ring, no vote per step), 2 the shared-memory-ring form
+ * (records copied ahead with cp.async, faster where most plane hand-offs cross thread-block
+ * clusters); all give the same bits.  DXG_ERR_ARG for 2 when it does not fit the grid.  No
+ * counterpart in the reference. */
 int dxg_set_lane_ring(dxg_ctx* ctx, int form);
 /* Limit of every bounded wait inside the ILU(0) sweeps, in seconds (default 0.5; at most
  * 60).  A wait that runs out ends the sweep with DXG_ERR_TIMEOUT, which the Newton driver
@@ -391,9 +395,10 @@ int dxg_batch_destroy(dxg_batch* batch);
 const char* dxg_batch_last_error(const dxg_batch* batch);
 /* DXG_BATCH_OPT_GRAPHS: replay the BiCGSTAB iterations of a solve from one captured
  * CUDA graph (default 1).  DXG_BATCH_OPT_AUTOTUNE: choose the cluster size, threads
- * and prefetch depth of the batched ILU(0) sweeps by timing candidates on the first
+ * and prefetch depth of the batched cluster-wavefront sweeps by timing candidates on the first
  * solve of each batch shape, kept for every batch of the process on that device
- * (default 1; 0 uses a fixed rule).  DXG_BATCH_OPT_ILU_REDBLACK:
+ * (default 1; 0 uses a fixed rule); a few problems together run the packed lane sweeps instead,
+ * which have nothing to tune.  DXG_BATCH_OPT_ILU_REDBLACK:
  * red-black ordered ILU(0) (as DXG_ILU_REDBLACK for a context) for every problem of the
  * batch (default 0, natural order); set before the first dxg_batch_add, else
  * DXG_ERR_STATE.  DXG_BATCH_OPT_AMG: AMG-BiCGSTAB (as DXG_LINEAR_SOLVER_AMG_BICGSTAB for a
@@ -403,7 +408,9 @@ int dxg_batch_set_option(dxg_batch* batch, int option, int value);
 /* Device memory that admitting this problem takes (tables and all solver state). */
 int64_t dxg_problem_device_bytes(const dxg_problem_desc* desc, int precision);
 /* Admission limit on the device memory of all admitted problems (0: unlimited).
- * dxg_batch_add refuses with DXG_ERR_BUDGET a problem that would exceed it. */
+ * dxg_batch_add refuses with DXG_ERR_BUDGET a problem that would exceed it.  The packed factor
+ * records of the natural-order sweeps (about another factor per problem) are no part of a
+ * problem's bytes; they are made within what a limit leaves and given back for admissions. */
 int dxg_batch_set_memory_budget(dxg_batch* batch, int64_t bytes);
 int64_t dxg_batch_device_bytes(const dxg_batch* batch);
 /* Admit a problem: initial solution u0 (N*num_eq values, also the first previous

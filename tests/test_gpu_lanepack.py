@@ -1,5 +1,7 @@
 """The lane sweeps over packed records against the cluster wavefront (the same arithmetic, so the
 same bits) at the edges of their tiles, warps and clusters, and their bounded waits."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -173,3 +175,38 @@ def test_packed_mpfa_plane_sweeps_wait_limit_expires_and_the_context_recovers():
     ctx.set_wait_limit(0.5)
     assert ctx.linear_solve(1e-10, 500)["iterations"] == first["iterations"]
     assert np.array_equal(ctx.update(), x0)
+
+
+def test_packed_sweeps_of_contexts_on_several_threads_equal_those_alone():
+    """Eight contexts whose sweeps need several clusters resident at once, solving at the same time
+    on streams of their own: no launch is held up half dispatched until its waits run out."""
+    def context(k):
+        if k % 4 == 3:
+            desc, u0 = problems.dnapl_2p_mpfa(cells=(16, 20, 16), seed=k)
+        else:
+            desc, u0 = problems.dnapl_2p(cells=(40, 48, 30), seed=k)
+        u = u0.reshape(-1, 2).copy()
+        u[:, 1] = np.random.default_rng(k).uniform(0.0, 0.4, len(u))
+        ctx = Context(desc, precision="fp64" if k % 2 else "mixed")
+        ctx.set_solution(u.reshape(-1))
+        ctx.set_prev_solution(u0)
+        ctx.set_time_step(250.0)
+        ctx.assemble_jacobian_and_residual()
+        return ctx
+
+    contexts = [context(k) for k in range(8)]
+    alone = [(c.linear_solve(1e-6, 400)["iterations"], c.update()) for c in contexts]
+    assert all("packed records" in c.describe() for c in contexts)
+    together = [None] * 8
+
+    def work(k):
+        for _ in range(5):
+            together[k] = (contexts[k].linear_solve(1e-6, 400)["iterations"], contexts[k].update())
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(alone, together):
+        assert b is not None and a[0] == b[0] and np.array_equal(a[1], b[1])
