@@ -329,6 +329,11 @@ __global__ void amgRestrictKernel(AmgLevel<T> F, AmgLevel<T> C, const KrylovStat
 constexpr int kAmgMaxClusterLevels = 12;
 constexpr int kAmgClusterCtas = 16;
 constexpr int kAmgClusterThreads = 512;
+// Largest second level, in cells.  A time step with the cluster launch from the level above it, and
+// from that level itself, against all small levels in one cluster launch out of global memory: FP64
+// 40x30x20 (second level of 400 cells) 42.5 and 38.6 ms against 43.9; FP32 41x30x20 (440) 23.9 and
+// 25.4 against 26.8, 70x58x8 (540) 15.9 and 16.3 against 16.4.
+constexpr int64_t kAmgOneCtaLevel64 = 256, kAmgOneCtaLevel32 = 640;
 constexpr size_t kAmgClusterSmem = 220 * 1024;
 template <class T>
 struct AmgCycle {
@@ -778,7 +783,10 @@ int64_t vcycle(const std::vector<AmgLevel<T>>& Ls, size_t l, const KrylovState* 
     const AmgLevel<T>& L = Ls[l];
     const unsigned g = gridFor(L.N);
     size_t elems = 0;
-    if (L.N <= kAmgClusterLevel && Ls.size() - l <= (size_t)kAmgMaxClusterLevels) {
+    // the level after the top one runs in one CTA: where it is large, in FP64 above all, a pass costs
+    // that SM more than a launch spread over the GPU, and the cluster starts a level further down
+    const bool oneCta = l + 1 >= Ls.size() || Ls[l + 1].N <= (sizeof(T) == 8 ? kAmgOneCtaLevel64 : kAmgOneCtaLevel32);
+    if (L.N <= kAmgClusterLevel && Ls.size() - l <= (size_t)kAmgMaxClusterLevels && oneCta) {
         const size_t last = Ls.size() - 1;
         elems = last > l ? amgTopElems<B, DIM, T>(L.N) : 0;
         for (size_t k = last > l ? l + 1 : l; k <= last; ++k) elems += amgSubElems<B, DIM, T>(Ls[k].N, k == last, false);
