@@ -1102,7 +1102,8 @@ def main():
         rnote = "bandwidth-bound passes, latency bound at small grids"
     elif args.workload in ("mpfa", "mpfa2p"):
         dsc = ctx.describe()
-        kname = (("stencilPlaneApply" if "one z-plane per CTA" in dsc else "stencilPackApply") if packed else
+        kname = (("stencilPlaneApply" if "one z-plane per CTA" in dsc else "stencilPackApply")
+                 if "packed records" in dsc else
                  "stencilLane3dKernel" if "one z-plane per CTA" in dsc else
                  "stencilLane2dKernel" if "over a cluster" in dsc else
                  "stencilWave2dKernel" if "line sweeps" in dsc else "stencilApplyKernel")
