@@ -33,9 +33,12 @@
 // the z history is used in both directions), so the turn costs no launch.
 // So a cluster waits for clusters of lower and of higher index, and a launch whose clusters are not
 // all resident would wait for itself: the plan counts them (cudaOccupancyMaxActiveClusters), a
-// batched launch takes no more problems than fit.  Launches of other streams only delay: a grid's
-// CTAs are dispatched whole before those of the next one (sixteen contexts solving on sixteen
-// threads ran without an expired wait).
+// batched launch takes no more problems than fit, and a launch of several clusters is a cooperative
+// one, which CUDA runs with all its CTAs resident whatever else the GPU is doing.  (The count
+// alone does not give that: placed around the CTAs of the kernel before it or of another stream,
+// the clusters leave gaps that no cluster fits.  4x4x700 cells, FP64 1x1: 88 clusters of 8 where
+// 89 fit, and the waits of a plain dependent launch expired.  The attribute costs nothing: 24
+// iterations on 64x64x32 FP64 take 7.52 ms either way.)
 // Every history starts filled with an all-ones pattern (a NaN that no arithmetic produces)
 // which the consumer waits to see replaced: each entry is one aligned 4- or 8-byte relaxed
 // store, seen whole, so no fence, flag or barrier sits on the chain.  The consumer puts the
@@ -617,15 +620,18 @@ cudaError_t lpLaunch(const LpShape& p, const LanePackArgs<T>& a, const LanePackA
     cfg.blockDim = dim3((p.warps + 1) * 32);
     cfg.dynamicSmemBytes = p.smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[3];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = p.clusterSize;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
+    // the clusters wait for one another: all of them resident
+    attr[2].id = cudaLaunchAttributeCooperative;
+    attr[2].val.cooperative = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = fits ? 1 : 2;
+    cfg.numAttrs = fits ? 1 : p.grid > (unsigned)p.clusterSize ? 3 : 2;
     if (fits) {
         int n = 0;
         e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);

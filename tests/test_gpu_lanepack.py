@@ -69,6 +69,61 @@ def test_packed_lane_sweeps_wait_limit_expires_and_the_context_recovers():
     assert np.array_equal(ctx.update(), x0)
 
 
+# all the clusters that fit the GPU at once, or nearly (88 of 8 CTAs, several CTAs per SM), and
+# clusters of odd sizes: every one of them has to be resident for the sweeps to end
+_CROWD = [(1, (4, 4, 700), "fp64"), (2, (24, 200, 24), "fp64"), (2, (64, 64, 90), "fp64"), (2, (45, 37, 23), "mixed"),
+          (1, (20, 20, 100), "fp64"), (2, (8, 8, 300), "fp64")]
+
+
+def _crowd_context(eqs, dims, precision, kind="auto"):
+    if eqs == 1:
+        desc, prev = problems.darcy_1p(cells=dims, seed=4)
+        u = prev
+    else:
+        desc, prev = problems.dnapl_2p(cells=dims, seed=4)
+        u = prev.reshape(-1, 2).copy()
+        u[:, 1] = np.random.default_rng(3).uniform(0.0, 0.3, len(u))
+        u = u.reshape(-1)
+    ctx = Context(desc, precision=precision)
+    ctx.set_ilu_kernel(kind)
+    ctx.set_solution(u)
+    if eqs == 2:
+        ctx.set_prev_solution(prev)
+        ctx.set_time_step(250.0)
+    ctx.assemble_jacobian_and_residual()
+    return ctx
+
+
+@pytest.mark.parametrize("eqs,dims,precision", _CROWD)
+def test_packed_sweeps_of_many_clusters_equal_cluster_wavefront(eqs, dims, precision):
+    ref = _crowd_context(eqs, dims, precision, "wavefront")
+    ctx = _crowd_context(eqs, dims, precision)
+    n0, n1 = (c.linear_solve(1e-4, 40)["iterations"] for c in (ref, ctx))
+    assert "packed records" in ctx.describe()
+    assert n1 == n0
+    assert np.array_equal(ctx.update(), ref.update())
+
+
+def test_packed_sweeps_of_clusters_of_many_sizes_on_several_threads():
+    """Launches that leave each other no room for all their clusters (88 clusters of 8 CTAs, 24 of
+    13, 6 of 15, 2 of 12, 7 of 15, 19 of 16), from streams of their own."""
+    contexts = [_crowd_context(*case) for case in _CROWD]
+    alone = [(c.linear_solve(1e-4, 40)["iterations"], c.update()) for c in contexts]
+    together = [None] * len(contexts)
+
+    def work(k):
+        for _ in range(5):
+            together[k] = (contexts[k].linear_solve(1e-4, 40)["iterations"], contexts[k].update())
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(contexts))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(alone, together):
+        assert b is not None and a[0] == b[0] and np.array_equal(a[1], b[1])
+
+
 # two warps of 32 lines per CTA (one on long lines); histories across warps, CTAs and remainders
 @pytest.mark.parametrize("cells", [(1, 1), (5, 4), (9, 31), (3, 33), (70, 64), (6, 65), (40, 130), (33, 257), (300, 40)])
 def test_packed_mpfa_sweeps_equal_level_kernel(cells):
