@@ -1,4 +1,4 @@
-// handoff.cuh -- what the packed lane sweeps (lanepack.cu, stencilpack.cu) share: hand-off
+// handoff.cuh -- what the packed lane sweeps (lanepack.cu, stencilpack.cu, stencilplane.cu) share: hand-off
 // histories polled for an all-ones pattern with bounded waits, record rings filled by bulk
 // copies, and asynchronous copies of vector entries.
 #pragma once
@@ -34,6 +34,18 @@ __device__ __forceinline__ bool lpIsEmpty(T v)
 {
     if constexpr (sizeof(T) == 8) return __double2hiint(v) == -1;
     else return __float_as_int(v) == -1;
+}
+// A factor entry for the sweeps.  A NaN keeps its bits through FP64 arithmetic (but for the sign), and
+// a caller's matrix may hold one with all bits set: the packed records hold another NaN in its place,
+// so no result ever looks like the pattern (a right-hand side with a NaN ends the solve before the
+// sweeps).  Told by the bits, off the FP64 pipe.
+__device__ __forceinline__ double lpEntry(double v)
+{
+    return (__double2hiint(v) & 0x7fffffff) == 0x7fffffff ? __longlong_as_double(0x7ff8000000000000ll) : v;
+}
+__device__ __forceinline__ float lpEntry(float v)
+{
+    return (__float_as_int(v) & 0x7fffffff) == 0x7fffffff ? __int_as_float(0x7fc00000) : v;
 }
 // The hand-off stores and polls carry no "memory" clobber: they need no order against the
 // step's other memory operations (a poll issued early sees the pattern and repeats).

@@ -175,11 +175,11 @@ __device__ __forceinline__ void lpPackSweep(const LanePackArgs<T>& a, int64_t fi
                     const T* row = (DIR > 0 ? a.Lf + ((int64_t)(DIM - 1 - ax) * a.N + i) * BB
                                             : a.A + ((int64_t)(DIM + 1 + ax) * a.N + i) * BB) + (p.r + r) * B;
 #pragma unroll
-                    for (int e = 0; e < B; ++e) out[(ax * R + r) * B + e] = row[e];
+                    for (int e = 0; e < B; ++e) out[(ax * R + r) * B + e] = lpEntry(row[e]);
                 }
                 if (DIR < 0)
 #pragma unroll
-                    for (int e = 0; e < B; ++e) out[(DIM * R + r) * B + e] = a.Dinv[i * BB + (p.r + r) * B + e];
+                    for (int e = 0; e < B; ++e) out[(DIM * R + r) * B + e] = lpEntry(a.Dinv[i * BB + (p.r + r) * B + e]);
             }
         }
         unsigned char* dst = a.pack[DIR > 0 ? 0 : 1] + rec * (NV * 32 * (int64_t)sizeof(T));

@@ -91,9 +91,9 @@ __global__ void __launch_bounds__(256) stencilPackKernel(StencilArgs a, StencilP
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int slot = fwd ? e : 8 - e;
-                if ((m >> slot) & 1u) v[e] = a.LU[(int64_t)slot * a.N + i];
+                if ((m >> slot) & 1u) v[e] = lpEntry(a.LU[(int64_t)slot * a.N + i]);
             }
-            if (!fwd) v[4] = a.Dinv[i];
+            if (!fwd) v[4] = lpEntry(a.Dinv[i]);
         }
         // values in pairs (16 bytes per lane), the last one alone
         double* dst = out + rec * (NV * 32);

@@ -115,9 +115,9 @@ __global__ void __launch_bounds__(256) stencilPlanePackKernel(StencilArgs a, Ste
             double val = 0.0;
             if (q < 13) {
                 const int slot = fwd ? q : 26 - q;
-                if ((m >> slot) & 1u) val = a.LU[((int64_t)slot * a.N + i) * (B * B) + r * B + c];
+                if ((m >> slot) & 1u) val = lpEntry(a.LU[((int64_t)slot * a.N + i) * (B * B) + r * B + c]);
             } else if (cell) {
-                val = a.Dinv[i * (B * B) + r * B + c];
+                val = lpEntry(a.Dinv[i * (B * B) + r * B + c]);
             }
             dst[NV * 8 % 16 != 0 && e == NV - 1 ? (NV - 1) * 32 + lane : (e / 2) * 64 + lane * 2 + e % 2] = val;
         }

@@ -5,7 +5,7 @@ import threading
 import numpy as np
 import pytest
 
-from dumux_gb300 import Batch, Context, newton_params, problem_device_bytes, problems
+from dumux_gb300 import Batch, Context, NumericalProblem, newton_params, problem_device_bytes, problems
 
 pytestmark = pytest.mark.gpu
 
@@ -265,3 +265,53 @@ def test_packed_sweeps_of_contexts_on_several_threads_equal_those_alone():
         t.join()
     for a, b in zip(alone, together):
         assert b is not None and a[0] == b[0] and np.array_equal(a[1], b[1])
+
+
+def _status(desc, u, dt, precision, kind, spoil):
+    ctx = Context(desc, precision=precision)
+    ctx.set_ilu_kernel(kind)
+    ctx.set_solution(u)
+    if dt:
+        ctx.set_prev_solution(u)
+        ctx.set_time_step(dt)
+    ctx.assemble_jacobian_and_residual()
+    rows, cols, values = ctx.jacobian()
+    rhs = ctx.residual()
+    spoil(rows, values, rhs)
+    ctx.set_linear_system(rows, cols, values, rhs)
+    with pytest.raises(NumericalProblem) as e:
+        ctx.linear_solve(1e-8, 100, raise_on_failure=True)
+    return e.value.status
+
+
+# what the sweeps wait for is a NaN with all bits set: neither that one in the caller's system nor
+# other values that are not finite may keep them waiting
+@pytest.mark.parametrize("value", [b"\xff" * 8, b"\xff" * 7 + b"\x7f", np.float64("nan").tobytes(),
+                                   np.float64("-inf").tobytes()], ids=["ones", "ones but the sign", "nan", "inf"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("disc,eqs,dims", [("tpfa", 1, (20, 30)), ("tpfa", 1, (9, 10, 20)), ("tpfa", 2, (20, 30)),
+                                           ("tpfa", 2, (9, 10, 20)), ("mpfa", 1, (20, 40)), ("mpfa", 1, (6, 33, 4)),
+                                           ("mpfa", 2, (6, 17, 4))])
+def test_values_that_are_not_finite_end_the_solve_as_on_the_other_kernels(disc, eqs, dims, precision, value):
+    if disc == "mpfa" and precision == "mixed":
+        pytest.skip("MPFA-O contexts solve in FP64")
+    dt = 250.0 if eqs == 2 else 0.0
+    if disc == "tpfa":
+        desc, u = (problems.darcy_1p(cells=dims, seed=4) if eqs == 1 else
+                   problems.dnapl_2p(cells=dims, extent=(6.0, 4.0, 1.0)[:len(dims)], seed=4))
+    elif eqs == 2:
+        desc, u = problems.dnapl_2p_mpfa(cells=dims, seed=4)
+    else:
+        K = ((2.0, 0.5), (0.5, 1.0)) if len(dims) == 2 else ((2.0, 0.3, 0.1), (0.3, 1.0, 0.2), (0.1, 0.2, 1.5))
+        desc, u, _ = problems.mpfa_linear_field_problem(cells=dims, K=K, spacing_seed=2)
+    x = np.frombuffer(value)[0]
+
+    def in_matrix(rows, values, rhs):
+        values[rows[len(rows) // 2] * eqs * eqs] = x
+
+    def in_rhs(rows, values, rhs):
+        rhs[len(rhs) // 3] = x
+
+    other = "wavefront" if disc == "tpfa" else "levels"
+    for spoil in (in_matrix, in_rhs):
+        assert (_status(desc, u, dt, precision, "auto", spoil) == _status(desc, u, dt, precision, other, spoil))
