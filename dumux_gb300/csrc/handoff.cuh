@@ -107,13 +107,15 @@ __device__ __forceinline__ LpVal<T, B> lpLdGpu(const T* p)
     return r;
 }
 
-// Looked at every 64 empty polls: whether the wait should go on.  False once the CTA's sweep
-// has stopped or when the wait's time is up (which records DXG_ERR_TIMEOUT and stops it).
-__device__ __noinline__ bool lpGoOn(unsigned long long* deadline, int* stop, int* err, unsigned long long waitNs)
+// Looked at after every 64 empty polls of a wait (n so far): whether it should go on.  False once the
+// CTA's sweep has stopped or when the wait's time is up (which records DXG_ERR_TIMEOUT and stops it).
+// The limit is each wait's own: the first look of a wait starts it.  (It is done here, off the
+// sweeps' path: a deadline set or cleared in lpPoll itself cost the FP64 sweeps 3%.)
+__device__ __noinline__ bool lpGoOn(int n, unsigned long long* deadline, int* stop, int* err, unsigned long long waitNs)
 {
     if (*(volatile int*)stop) return false;
     const unsigned long long now = lpTimer();
-    if (*deadline == 0) *deadline = now + waitNs;
+    if (n == 64) *deadline = now + waitNs;
     else if (now > *deadline) {
         atomicExch(err, DXG_ERR_TIMEOUT);
         *(volatile int*)stop = 1;
@@ -130,7 +132,7 @@ __device__ __forceinline__ void lpPoll(LpVal<T, B>& r, LOAD&& load, unsigned lon
     int n = 0;
     while (__any_sync(0xffffffffu, r.empty())) {
         if ((++n & 63) == 0) {
-            const bool on = lpGoOn(deadline, stop, err, waitNs);
+            const bool on = lpGoOn(n, deadline, stop, err, waitNs);
             if (__any_sync(0xffffffffu, !on)) {
 #pragma unroll
                 for (int e = 0; e < B; ++e) r.v[e] = 0;

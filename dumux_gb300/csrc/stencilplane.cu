@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kPlRoles * kPlMaxTiles * 32) stencilPlaneApply
             int n = 0;
             while (__any_sync(0xffffffffu, busy())) {
                 if ((++n & 63) == 0) {
-                    const bool on = lpGoOn(deadline, &stopFlag, a.err, waitNs);
+                    const bool on = lpGoOn(n, deadline, &stopFlag, a.err, waitNs);
                     if (__any_sync(0xffffffffu, !on)) return false;
                 }
                 again();

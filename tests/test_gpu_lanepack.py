@@ -315,3 +315,31 @@ def test_values_that_are_not_finite_end_the_solve_as_on_the_other_kernels(disc, 
     other = "wavefront" if disc == "tpfa" else "levels"
     for spoil in (in_matrix, in_rhs):
         assert (_status(desc, u, dt, precision, "auto", spoil) == _status(desc, u, dt, precision, other, spoil))
+
+
+@pytest.mark.parametrize("kind,limit", [("lanes", 90e-6), ("mpfa lines", 130e-6), ("mpfa planes", 120e-6)])
+def test_wait_limit_is_that_of_a_single_wait(kind, limit):
+    """Long lines: a launch takes 260 to 330 us, and the warps of its middle planes (lines) wait twice, at
+    the start and at the turn, no wait being longer than about 80 us.  The limit is above every single
+    wait and below the time between the two."""
+    if kind == "mpfa lines":
+        desc, u, _ = problems.mpfa_linear_field_problem(cells=(600, 128), spacing_seed=3)
+        prev, dt = u, 0.0
+    else:
+        desc, prev = (problems.dnapl_2p(cells=(300, 16, 40), seed=8) if kind == "lanes" else
+                      problems.dnapl_2p_mpfa(cells=(200, 10, 16), seed=8))
+        u = prev.reshape(-1, 2).copy()
+        u[:, 1] = np.random.default_rng(5).uniform(0.0, 0.4, len(u))
+        u, dt = u.reshape(-1), 250.0
+    ctx = Context(desc)
+    ctx.set_solution(u)
+    if dt:
+        ctx.set_prev_solution(prev)
+        ctx.set_time_step(dt)
+    ctx.assemble_jacobian_and_residual()
+    first = ctx.linear_solve(1e-6, 60)
+    assert "packed records" in ctx.describe()
+    x0 = ctx.update()
+    ctx.set_wait_limit(limit)
+    assert ctx.linear_solve(1e-6, 60) == first
+    assert np.array_equal(ctx.update(), x0)
