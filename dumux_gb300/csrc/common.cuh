@@ -86,7 +86,8 @@ struct DevBuf {
 // A launch of the Krylov iteration's chain: a programmatic dependent of the launch before it, whose
 // blocks may start (and stop in chainWait) while that one still runs, so its launch latency and
 // the ramp of the grid overlap with it.  Every kernel launched this way calls chainWait before it
-// touches memory.
+// touches memory, and reads what the chain writes with plain loads (the read-only path, __ldg or a
+// const __restrict__ parameter, is for data that nobody writes while the kernel runs).
 template <class... P, class... Q>
 inline void launchChained(void (*kern)(P...), dim3 grid, unsigned threads, cudaStream_t st, Q&&... args)
 {

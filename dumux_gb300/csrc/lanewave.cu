@@ -369,7 +369,8 @@ __global__ void __launch_bounds__(kLwThreads) laneWaveKernel(LaneWaveArgs<T> a)
         rY[k] = act && hasY ? lwLdg2(srcY + 4 * x) : zero;
         rZ[k] = act && hasZ ? lwLdg2(srcZ + 4 * x) : zero;
         if (DIR < 0) rD[k] = act ? lwLdg2(srcD + 4 * x) : zero;
-        rV[k] = act ? __ldg(srcV + 2 * x) : T(0);
+        // (a plain load: the backward sweep starts while the forward one still writes)
+        rV[k] = act ? srcV[2 * x] : T(0);
     };
 
     const bool warpWorks = working && !skip && sy0 + warp * kLwLinesPerWarp < ny;

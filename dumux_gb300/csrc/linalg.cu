@@ -184,9 +184,11 @@ __device__ __forceinline__ void storeVec(T* p, int64_t i, const T* v)
     for (int e = 0; e < B; ++e) p[i * B + e] = v[e];
 }
 
-// Read-only vector loads of one b x b block / one b-vector (16-byte loads for 2 x 2 FP32
-// blocks and FP64 pairs; every block and vector entry starts on a multiple of its size
-// from a cudaMalloc base).  Only for data no kernel writes while the reader runs.
+// Vector loads of one b x b block / one b-vector (16-byte loads for 2 x 2 FP32 blocks and FP64
+// pairs; every block and vector entry starts on a multiple of its size from a cudaMalloc base).
+// Blocks through the read-only path: the matrix and its pivots are finished before the chain of
+// Krylov kernels starts.  Vectors not: the launch before may still be writing them when this one
+// has started, and only plain loads are ordered by chainWait.
 template <int B, class T>
 __device__ __forceinline__ void ldgBlock(const T* p, T* o)
 {
@@ -203,17 +205,17 @@ __device__ __forceinline__ void ldgBlock(const T* p, T* o)
     }
 }
 template <int B, class T>
-__device__ __forceinline__ void ldgVec(const T* p, T* o)
+__device__ __forceinline__ void ldVec(const T* p, T* o)
 {
     if constexpr (B == 2 && sizeof(T) == 4) {
-        const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+        const float2 v = *reinterpret_cast<const float2*>(p);
         o[0] = v.x; o[1] = v.y;
     } else if constexpr (B == 2 && sizeof(T) == 8) {
-        const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+        const double2 v = *reinterpret_cast<const double2*>(p);
         o[0] = v.x; o[1] = v.y;
     } else {
 #pragma unroll
-        for (int e = 0; e < B; ++e) o[e] = __ldg(p + e);
+        for (int e = 0; e < B; ++e) o[e] = p[e];
     }
 }
 
@@ -276,7 +278,7 @@ __global__ void __launch_bounds__(kReduceThreads, 4) spmvKernel(SpmvArgs<MT, VT,
             MT blk[BB];
             XT xs[B];
             ldgBlock<B>(a.A + ((int64_t)s * a.N + i) * BB, blk);
-            ldgVec<B>(a.x + (i + (valid ? a.off[s] : 0)) * B, xs);
+            ldVec<B>(a.x + (i + (valid ? a.off[s] : 0)) * B, xs);
             AT xj[B];
 #pragma unroll
             for (int e = 0; e < B; ++e) {
@@ -481,7 +483,7 @@ __global__ void rbApplyBlack(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* 
     unsigned lb;
     const RbArgs<T> a = problemOf(a0, batch, map, lb);
     if (a.ks && a.ks->status != KS_RUNNING) return;
-    const T* __restrict__ d = a.d;
+    const T* d = a.d;
     T* __restrict__ v = a.v;
     constexpr int BB = B * B, S = 2 * DIM + 1;
     const int64_t rows = (int64_t)a.ny * a.nz, total = rows * ((a.nx + 1) / 2);
@@ -492,7 +494,7 @@ __global__ void rbApplyBlack(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* 
         if (i < 0) continue;
         const unsigned m = __ldg(a.nbmask + i);
         T acc[B];
-        ldgVec<B>(d + i * B, acc);
+        ldVec<B>(d + i * B, acc);
         // FP32: straight-line loads of every neighbour slot (the cell's own entries stand in
         // for a missing neighbour, whose block enters as zero), so all gathers are in flight
         // together; FP64 skips missing neighbours (its zero products would cost FP64 issue)
@@ -505,7 +507,7 @@ __global__ void rbApplyBlack(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* 
             T Aij[BB], Dj[BB], dj[B], w[B];
             ldgBlock<B>(a.A + ((int64_t)s * a.N + i) * BB, Aij);
             ldgBlock<B>(a.Dinv + j * BB, Dj);
-            ldgVec<B>(d + j * B, dj);
+            ldVec<B>(d + j * B, dj);
 #pragma unroll
             for (int e = 0; e < BB; ++e) Aij[e] = valid ? Aij[e] : (T)0;
 #pragma unroll
@@ -533,7 +535,7 @@ __global__ void rbApplyRed(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* ma
     unsigned lb;
     const RbArgs<T> a = problemOf(a0, batch, map, lb);
     if (a.ks && a.ks->status != KS_RUNNING) return;
-    const T* __restrict__ d = a.d;
+    const T* d = a.d;
     T* v = a.v;
     constexpr int BB = B * B, S = 2 * DIM + 1;
     const int64_t rows = (int64_t)a.ny * a.nz, total = rows * ((a.nx + 1) / 2);
@@ -544,7 +546,7 @@ __global__ void rbApplyRed(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* ma
         if (i < 0) continue;
         const unsigned m = __ldg(a.nbmask + i);
         T acc[B];
-        ldgVec<B>(d + i * B, acc);
+        ldVec<B>(d + i * B, acc);
 #pragma unroll
         for (int s = 0; s < S; ++s) {
             if (s == DIM) continue;
@@ -1194,8 +1196,8 @@ template void launchCopyToDouble<float>(const float*, double*, int64_t, cudaStre
 // y = A x; MODE 1: also dot(w, y) -> h, alpha; MODE 2: dots (y,w),(y,y) -> omega (the
 // Krylov-state updates of spmvKernel)
 template <int S, int MODE>
-__global__ void __launch_bounds__(kReduceThreads) stencilSpmvKernel(StencilArgs a, const double* __restrict__ x,
-                                                                     double* __restrict__ y, const double* __restrict__ w)
+__global__ void __launch_bounds__(kReduceThreads) stencilSpmvKernel(StencilArgs a, const double* x, double* __restrict__ y,
+                                                                     const double* w)
 {
     chainWait();
     const unsigned nblk = cellBlocksFor(a.N);
@@ -1209,7 +1211,7 @@ __global__ void __launch_bounds__(kReduceThreads) stencilSpmvKernel(StencilArgs 
         for (int s = 0; s < S; ++s) {
             const bool valid = (m >> s) & 1u;
             const double aij = __ldg(a.A + (int64_t)s * a.N + i);
-            const double xj = __ldg(x + i + (valid ? a.off[s] : 0));
+            const double xj = x[i + (valid ? a.off[s] : 0)];
             sum += valid ? aij * xj : 0.0;
         }
         y[i] = sum;
@@ -1426,8 +1428,8 @@ __global__ void __launch_bounds__(MAXT) stencilWave2dKernel(StencilArgs a, const
 // blocks): SpMV with the same fused dots, and the block ILU(0) factor and sweeps level by
 // level (block products with explicit FMAs, pivot blocks inverted as in the wavefront factor)
 template <int S, int MODE>
-__global__ void __launch_bounds__(kReduceThreads) stencilSpmv2Kernel(StencilArgs a, const double* __restrict__ x,
-                                                                      double* __restrict__ y, const double* __restrict__ w)
+__global__ void __launch_bounds__(kReduceThreads) stencilSpmv2Kernel(StencilArgs a, const double* x, double* __restrict__ y,
+                                                                      const double* w)
 {
     chainWait();
     const unsigned nblk = cellBlocksFor(a.N);
@@ -1442,7 +1444,7 @@ __global__ void __launch_bounds__(kReduceThreads) stencilSpmv2Kernel(StencilArgs
             const bool valid = (m >> s) & 1u;
             double blk[4], xs[2];
             ldgBlock<2>(a.A + ((int64_t)s * a.N + i) * 4, blk);
-            ldgVec<2>(x + (i + (valid ? a.off[s] : 0)) * 2, xs);
+            ldVec<2>(x + (i + (valid ? a.off[s] : 0)) * 2, xs);
 #pragma unroll
             for (int e = 0; e < 2; ++e) xs[e] = valid ? xs[e] : 0.0;
 #pragma unroll

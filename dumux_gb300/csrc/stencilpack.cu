@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256) stencilPackKernel(StencilArgs a, StencilP
 }
 
 __global__ void __launch_bounds__((kSpMaxWarps + 1) * 32) stencilPackApply(StencilArgs a, StencilPackPlan pl,
-                                                                            const double* __restrict__ d, double* v)
+                                                                            const double* d, double* v)
 {
     constexpr int SS = kSpStageSteps, STAGE = SS * kSpBwd * 32 * 8, LPW = kSpLines;
     extern __shared__ __align__(128) unsigned char spRaw[];

@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(256) stencilPlanePackKernel(StencilArgs a, Ste
 
 template <int B>
 __global__ void __launch_bounds__(kPlRoles * kPlMaxTiles * 32) stencilPlaneApply(StencilArgs a, StencilPlanePlan pl,
-                                                                               const double* __restrict__ d, double* v)
+                                                                               const double* d, double* v)
 {
     using Val = LpVal<double, B>;
     constexpr int LPW = 32 / B, SS = kPlStageSteps, REC1 = B * 32 * 8;   // bytes of one term of a record
