@@ -598,7 +598,7 @@ void tabulate(dxg_ctx* c, const dxg_problem_desc* d)
     c->packPlan = LanePackPlan{};
     c->stencilPack = StencilPackPlan{};
     c->stencilPlane = StencilPlanePlan{};
-    c->packPlanned = false;
+    c->packPlanned = c->packTimed = false;
     c->packMem.release();
     c->waveTuneCount = 0;
     c->dropGraphs();   // the captured chunks hold the old buffers' addresses
@@ -769,7 +769,7 @@ void tabulateMpfa(dxg_ctx* c, const dxg_problem_desc* d)
     c->packPlan = LanePackPlan{};
     c->stencilPack = StencilPackPlan{};
     c->stencilPlane = StencilPlanePlan{};
-    c->packPlanned = false;
+    c->packPlanned = c->packTimed = false;
     c->packMem.release();
     c->waveTuneCount = 0;
     c->dropGraphs();
@@ -1149,6 +1149,14 @@ LaneWaveArgs<T> laneArgs(dxg_ctx* c, const T* A, const T* L, const T* Dinv, cons
 // 0.129 ms per apply against 0.195 ms for the register form and 0.345 ms for the cluster
 // wavefront, in FP32 0.068, 0.156 and 0.207 ms; 2D 100x100 1x1 0.056 ms against 0.097 ms for the
 // one-CTA line sweeps and 0.193 ms, 10x10 0.0085 against 0.015 and 0.023 ms).
+// A plan of many clusters is not always the better one where the lane sweeps that read the factor in
+// place fit, too (3D, 2x2 blocks): these put more lines on a CTA, so they hand on between fewer
+// clusters.  Up to eight clusters the packed sweeps were faster on each of some 250 grids timed (by 2%
+// at least: 8x8x128 FP64), without such a competitor on all; beyond eight, 16 iterations took, in ms
+// against the register form: 8x8x200 FP64 (13 clusters) 6.2 and 6.0, 24x200x24 FP64 (24) 10.9 and 12.0,
+// 5x33x128 mixed (32) 6.5 and 4.2, 128x128x64 mixed (32) 14.8 and 21.9, 4x4x400 mixed (50) 9.3 and 7.5.
+// So those are timed at the first factorisation, as the other kernels are.
+constexpr int kPackSureClusters = 8;
 bool usePack(const dxg_ctx* c)
 {
     return c->packPlan.ok && c->laneRingMode == 0 && c->linearSolver == DXG_LINEAR_SOLVER_ILU_BICGSTAB &&
@@ -1164,6 +1172,7 @@ void preparePack(dxg_ctx* c)
         c->packPlanned = true;
         c->packPlan = makeLanePackPlan<T>(c->dim, (int)c->pcHost.nx, (int)c->pcHost.ny, c->dim == 3 ? (int)c->pcHost.nz : 1,
                                           c->b);
+        c->packTimed = c->packPlan.ok && c->lanePlan.ok && c->packPlan.grid > kPackSureClusters * c->packPlan.clusterSize;
     }
     if (!usePack(c) || c->packMem.get()) return;
     const LanePackPlan& p = c->packPlan;
@@ -1272,7 +1281,7 @@ std::vector<AmgLevel<T>> amgLevels(dxg_ctx* c, const T* A, T* Dinv, const T* in,
     return L;
 }
 
-// Launch shape of the wavefront sweeps, chosen once per context by timing: every plan
+// Launch shape of the natural-order sweeps, chosen once per context by timing: every wavefront plan
 // that fits (cluster sizes 16..1) applies the preconditioner built by the first
 // factorisation to `in` (a scratch read) into `out` (overwritten by the solve that
 // follows); the fastest is kept.  Small grids run faster on fewer CTAs (fewer hand-offs
@@ -1367,6 +1376,24 @@ void tuneWavePlan(dxg_ctx* c, const T* A, T* L, T* Dinv, const T* in, T* out)
         ms /= kReps;
         c->line2dMs = ms;
         c->line2d = bestMs == 0.f || ms < bestMs;
+    }
+    // the packed lane sweeps, where their plan leaves it open (packTimed)
+    if (usePack(c)) {
+        LanePackArgs<T> pa = packArgs<T>(c, A, L, Dinv, in, out);
+        pa.ks = nullptr;   // never skip while timing
+        launchLanePackApply<T>(c->packPlan, pa, st);   // warm-up
+        DXG_CUDA(cudaEventRecord(e0, st));
+        for (int r = 0; r < kReps; ++r) launchLanePackApply<T>(c->packPlan, pa, st);
+        DXG_CUDA(cudaEventRecord(e1, st));
+        DXG_CUDA(cudaEventSynchronize(e1));
+        c->launches += 1 + kReps;
+        float ms = 0.f;
+        DXG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        ms /= kReps;
+        if ((useLane(c) && ms > c->laneTuneMs) || (c->iluKernel == DXG_ILU_AUTO && bestMs > 0.f && ms > bestMs)) {
+            c->packPlan.ok = false;
+            c->packMem.release();
+        }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -1504,7 +1531,7 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
     sv.ks = c->ks.get();
     sv.scratch = c->scratch();
     const bool amg = c->linearSolver == DXG_LINEAR_SOLVER_AMG_BICGSTAB;
-    if (refactor && !amg && useWave(c) && !c->waveTuned && !usePack(c)) tuneWavePlan<PT>(c, PA, PL, PD, pIn, yOut);
+    if (refactor && !amg && useWave(c) && !c->waveTuned && (!usePack(c) || c->packTimed)) tuneWavePlan<PT>(c, PA, PL, PD, pIn, yOut);
     std::vector<AmgLevel<PT>> amgP, amgR;
     if (amg) {
         amgP = amgLevels<PT>(c, PA, PD, pIn, yOut);

@@ -124,6 +124,7 @@ struct dxg_ctx {
     dxg::StencilPackPlan stencilPack;     // ... and of the 2D scalar MPFA-O stencil
     dxg::StencilPlanePlan stencilPlane;   // ... and of the 3D one
     bool packPlanned = false;
+    bool packTimed = false;               // the TPFA plan is timed against the others at the first factorisation
     dxg::DevBuf<unsigned char> packMem;   // records of both sweeps, then the hand-off buffer
     dxg::DevBuf<unsigned char> laneHandoff;
     size_t laneHandoffBytes = 0;

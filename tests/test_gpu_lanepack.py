@@ -71,7 +71,7 @@ def test_packed_lane_sweeps_wait_limit_expires_and_the_context_recovers():
 
 # all the clusters that fit the GPU at once, or nearly (88 of 8 CTAs, several CTAs per SM), and
 # clusters of odd sizes: every one of them has to be resident for the sweeps to end
-_CROWD = [(1, (4, 4, 700), "fp64"), (2, (24, 200, 24), "fp64"), (2, (64, 64, 90), "fp64"), (2, (45, 37, 23), "mixed"),
+_CROWD = [(1, (4, 4, 700), "fp64"), (1, (24, 200, 24), "fp64"), (2, (64, 64, 90), "fp64"), (2, (45, 37, 23), "mixed"),
           (1, (20, 20, 100), "fp64"), (2, (8, 8, 300), "fp64")]
 
 
@@ -104,9 +104,24 @@ def test_packed_sweeps_of_many_clusters_equal_cluster_wavefront(eqs, dims, preci
     assert np.array_equal(ctx.update(), ref.update())
 
 
+def test_packed_sweeps_of_many_clusters_give_way_to_faster_ones():
+    """256 CTAs in 32 clusters of 8 take 1.5 times as long as the lane sweeps that read the factor in
+    place from 8 clusters of 16: the timing at the first factorisation finds out."""
+    ref, ctx, lanes = (_crowd_context(2, (5, 33, 128), "mixed", kind) for kind in ("wavefront", "auto", "lanes"))
+    n0 = ref.linear_solve(1e-4, 40)["iterations"]
+    for c in (ctx, lanes):
+        assert c.linear_solve(1e-4, 40)["iterations"] == n0
+        assert "packed records" not in c.describe()
+        assert np.array_equal(c.update(), ref.update())
+    # the records are given back, and another solve of the same context does without them
+    ctx.assemble_jacobian_and_residual()
+    assert ctx.linear_solve(1e-4, 40)["iterations"] == n0
+    assert np.array_equal(ctx.update(), ref.update())
+
+
 def test_packed_sweeps_of_clusters_of_many_sizes_on_several_threads():
-    """Launches that leave each other no room for all their clusters (88 clusters of 8 CTAs, 24 of
-    13, 6 of 15, 2 of 12, 7 of 15, 19 of 16), from streams of their own."""
+    """Launches that leave each other no room for all their clusters (88 clusters of 8 CTAs, 5 of
+    15, 6 of 15, 2 of 12, 7 of 15, 19 of 16), from streams of their own."""
     contexts = [_crowd_context(*case) for case in _CROWD]
     alone = [(c.linear_solve(1e-4, 40)["iterations"], c.update()) for c in contexts]
     together = [None] * len(contexts)
