@@ -288,7 +288,7 @@ __device__ __forceinline__ void coarseRow(const AmgLevel<T>& L, int n, int i)
 template <int B, class T>
 __global__ void amgFirstKernel(AmgLevel<T> L, T* out, T omega, const KrylovState* ks)
 {
-    chainWait();
+    chainWait(kEarlyWide);
     if (stopped<T>(ks)) return;
     AMG_LOOP(L) firstCell<B, T>(L, i, out, omega);
 }
@@ -297,7 +297,7 @@ template <int B, int DIM, class T>
 __global__ void amgJacobiKernel(AmgLevel<T> L, const T* xin, const T* xc, int cnx, int cny, T* out, T omega,
                                 const KrylovState* ks)
 {
-    chainWait();
+    chainWait(kEarlyWide);
     if (stopped<T>(ks)) return;
     AMG_LOOP(L) jacobiCell<B, DIM, T>(L, i, xin, xc, cnx, cny, out, omega);
 }
@@ -305,7 +305,7 @@ __global__ void amgJacobiKernel(AmgLevel<T> L, const T* xin, const T* xc, int cn
 template <int B, int DIM, class T>
 __global__ void amgResidualKernel(AmgLevel<T> L, const T* xin, const KrylovState* ks)
 {
-    chainWait();
+    chainWait(kEarlyWide);
     if (stopped<T>(ks)) return;
     AMG_LOOP(L) residualCell<B, DIM, T>(L, i, xin);
 }
@@ -313,7 +313,7 @@ __global__ void amgResidualKernel(AmgLevel<T> L, const T* xin, const KrylovState
 template <int B, int DIM, class T>
 __global__ void amgRestrictKernel(AmgLevel<T> F, AmgLevel<T> C, const KrylovState* ks)
 {
-    chainWait();
+    chainWait(kEarlyWide);
     if (stopped<T>(ks)) return;
     AMG_LOOP(C) restrictCell<B, DIM, T>(F, C, i);
 }
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(kAmgClusterThreads) amgClusterCycle(AmgCycle<T
     const int first = rank * cpc, mine = max(0, min(cpc, N - first));
     // One decision for the whole cluster: a CTA must not leave while another reads its shared memory.
     __shared__ int stop;
-    chainWait();
+    chainWait(kEarlyWide);
     if (tid == 0) stop = ks ? __ldcg(&ks->status) != KS_RUNNING : 0;
     cl.sync();
     const int stopAll = *cl.map_shared_rank(&stop, 0);
@@ -728,7 +728,7 @@ __global__ void amgCoarseInvertKernel(AmgLevel<T> L, int* singular)
 template <class T>
 __global__ void amgCoarseSolveKernel(AmgLevel<T> L, int n, const KrylovState* ks)
 {
-    chainWait();
+    chainWait(kEarlyWide);
     if (stopped<T>(ks)) return;
     for (int i = threadIdx.x; i < n; i += blockDim.x) coarseRow<T>(L, n, i);
 }

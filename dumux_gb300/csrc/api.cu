@@ -1531,6 +1531,7 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
     sv.ks = c->ks.get();
     sv.scratch = c->scratch();
     const bool amg = c->linearSolver == DXG_LINEAR_SOLVER_AMG_BICGSTAB;
+    ba.early = sv.early = amg || c->iluKernel == DXG_ILU_REDBLACK ? kEarlyWide : kEarlySweep;
     if (refactor && !amg && useWave(c) && !c->waveTuned && (!usePack(c) || c->packTimed)) tuneWavePlan<PT>(c, PA, PL, PD, pIn, yOut);
     std::vector<AmgLevel<PT>> amgP, amgR;
     if (amg) {

@@ -1122,8 +1122,9 @@ GroupState& groupState(dxg_batch* B, const GroupKey& key, const Members& S)
         G.classes[q].dBw = d + oc[q][2];
     }
     G.dTd = reinterpret_cast<const ToDoubleArgs*>(d + oT);
-    G.mapM = {reinterpret_cast<const uint2*>(d + oM), (unsigned)mM.size()};
-    G.mapN = {reinterpret_cast<const uint2*>(d + oN), (unsigned)mN.size()};
+    const unsigned early = B->redBlack || B->amg ? kEarlyWide : kEarlySweep;
+    G.mapM = {reinterpret_cast<const uint2*>(d + oM), (unsigned)mM.size(), early};
+    G.mapN = {reinterpret_cast<const uint2*>(d + oN), (unsigned)mN.size(), early};
     G.mapH = {reinterpret_cast<const uint2*>(d + oH), (unsigned)mH.size()};
     G.dRbP = d + oRP;
     G.dRbR = d + oRR;

@@ -102,13 +102,22 @@ inline void launchChained(void (*kern)(P...), dim3 grid, unsigned threads, cudaS
     cfg.numAttrs = 1;
     DXG_CUDA(cudaLaunchKernelEx(&cfg, kern, std::forward<Q>(args)...));
 }
-// Waits until the launch before has completed and its writes are visible.  A grid of at most one
-// block per SM lets the next launch of the chain start at once; of a larger one that would take
-// room on the SMs from its own blocks (measured per BiCGSTAB iteration with and without: 10x10
-// 34 / 39 us, 100x100 141 / 147 us, but 64x64x32 with the red-black sweeps 91 / 68 us).
-__device__ __forceinline__ void chainWait()
+// Waits until the launch before has completed and its writes are visible.  A grid of at most `early`
+// blocks lets the next launch of the chain start at once.  Its blocks then wait on the SMs that this
+// grid leaves free, several to an SM, and share that SM's FP64 pipe when they run; so how large a
+// grid may be depends on what follows:
+//   * a kernel over the whole GPU (red-black passes, AMG levels): a quarter of the SMs.  Sixteen
+//     iterations, never early, early up to 38 and up to 152 blocks: red-black 10x10 mixed 645, 595 and
+//     592 us, 24x24x24 FP64 929, 921 and 1011 us, 33x33x33 961, 961 and 1341 us; AMG 30x30x30 2771,
+//     2806 and 3750 us;
+//   * a cluster sweep, which has few CTAs and needs SMs of its own: up to one block per SM.  24x24x24
+//     FP64, never early, up to 38 and up to 152 blocks: 2371, 2322 and 2306 us, 32x32x32 mixed 2090,
+//     2090 and 2038 us.
+constexpr unsigned kSms = 152;   // of a GB300
+constexpr unsigned kEarlyWide = kSms / 4, kEarlySweep = kSms;
+__device__ __forceinline__ void chainWait(unsigned early)
 {
-    if (gridDim.x * gridDim.y <= 152u) asm volatile("griddepcontrol.launch_dependents;");
+    if (gridDim.x * gridDim.y <= early) asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 

@@ -253,7 +253,7 @@ template <int B, int DIM, class MT, class VT, class XT, int MODE>
 __global__ void __launch_bounds__(kReduceThreads, 4) spmvKernel(SpmvArgs<MT, VT, XT> a0,
                                                               const SpmvArgs<MT, VT, XT>* batch, const uint2* map)
 {
-    chainWait();
+    chainWait(a0.early);
     // accumulation: FP32 when both operands are FP32, else the output type
     using AT = typename std::conditional<sizeof(MT) == 4 && sizeof(XT) == 4, float, VT>::type;
     unsigned lb;
@@ -479,7 +479,7 @@ __global__ void rbFactorBlack(RbArgs<T> a0, const RbArgs<T>* batch, const uint2*
 template <int B, int DIM, class T>
 __global__ void rbApplyBlack(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* map)
 {
-    chainWait();
+    chainWait(kEarlyWide);
     unsigned lb;
     const RbArgs<T> a = problemOf(a0, batch, map, lb);
     if (a.ks && a.ks->status != KS_RUNNING) return;
@@ -531,7 +531,7 @@ __global__ void rbApplyBlack(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* 
 template <int B, int DIM, class T>
 __global__ void rbApplyRed(RbArgs<T> a0, const RbArgs<T>* batch, const uint2* map)
 {
-    chainWait();
+    chainWait(kEarlyWide);
     unsigned lb;
     const RbArgs<T> a = problemOf(a0, batch, map, lb);
     if (a.ks && a.ks->status != KS_RUNNING) return;
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(kReduceThreads) bicgInit(BicgArgs<VT> a0, cons
 template <class VT>
 __global__ void bicgUpdateP(BicgArgs<VT> a0, const BicgArgs<VT>* batch, const uint2* map)
 {
-    chainWait();
+    chainWait(a0.early);
     DXG_PROBLEM_BLOCKS(BicgArgs<VT>, M)
     const KrylovState& ks = *a.ks;
     if (ks.status != KS_RUNNING) return;
@@ -712,7 +712,7 @@ __global__ void bicgUpdateP(BicgArgs<VT> a0, const BicgArgs<VT>* batch, const ui
 template <class VT, int STAGE>
 __global__ void __launch_bounds__(kReduceThreads) bicgAxpyNorm(BicgArgs<VT> a0, const BicgArgs<VT>* batch, const uint2* map)
 {
-    chainWait();
+    chainWait(a0.early);
     DXG_PROBLEM_BLOCKS(BicgArgs<VT>, M)
     const KrylovState& ksr = *a.ks;
     if (ksr.status != KS_RUNNING) return;
@@ -925,7 +925,9 @@ template <class MT, class VT, class XT>
 void launchSpmvBatch(const SpmvArgs<MT, VT, XT>* batch, const BlockMap& cellMap, int b, int dim, int mode,
                      cudaStream_t st)
 {
-    spmvDispatch<MT, VT, XT>(SpmvArgs<MT, VT, XT>{}, batch, cellMap.map, dim3(cellMap.blocks), b, dim, mode, st);
+    SpmvArgs<MT, VT, XT> a0{};
+    a0.early = cellMap.early;
+    spmvDispatch<MT, VT, XT>(a0, batch, cellMap.map, dim3(cellMap.blocks), b, dim, mode, st);
 }
 
 template <class MT>
@@ -1055,13 +1057,17 @@ void launchBicgInitBatch(const BicgArgs<VT>* batch, const BlockMap& m, cudaStrea
 template <class VT>
 void launchBicgUpdatePBatch(const BicgArgs<VT>* batch, const BlockMap& m, cudaStream_t st)
 {
-    launchChained(bicgUpdateP<VT>, dim3(m.blocks), kReduceThreads, st, BicgArgs<VT>{}, batch, m.map);
+    BicgArgs<VT> a0{};
+    a0.early = m.early;
+    launchChained(bicgUpdateP<VT>, dim3(m.blocks), kReduceThreads, st, a0, batch, m.map);
 }
 template <class VT>
 void launchBicgAxpyNormBatch(const BicgArgs<VT>* batch, const BlockMap& m, int stage, cudaStream_t st)
 {
-    if (stage == 0) launchChained(bicgAxpyNorm<VT, 0>, dim3(m.blocks), kReduceThreads, st, BicgArgs<VT>{}, batch, m.map);
-    else launchChained(bicgAxpyNorm<VT, 1>, dim3(m.blocks), kReduceThreads, st, BicgArgs<VT>{}, batch, m.map);
+    BicgArgs<VT> a0{};
+    a0.early = m.early;
+    if (stage == 0) launchChained(bicgAxpyNorm<VT, 0>, dim3(m.blocks), kReduceThreads, st, a0, batch, m.map);
+    else launchChained(bicgAxpyNorm<VT, 1>, dim3(m.blocks), kReduceThreads, st, a0, batch, m.map);
 }
 template <class VT>
 void launchCopyToDouble(const VT* x, double* y, int64_t M, cudaStream_t st)
@@ -1199,7 +1205,7 @@ template <int S, int MODE>
 __global__ void __launch_bounds__(kReduceThreads) stencilSpmvKernel(StencilArgs a, const double* x, double* __restrict__ y,
                                                                      const double* w)
 {
-    chainWait();
+    chainWait(kEarlySweep);
     const unsigned nblk = cellBlocksFor(a.N);
     const unsigned lb = blockIdx.x;
     if (a.ks && a.ks->status != KS_RUNNING) return;
@@ -1431,7 +1437,7 @@ template <int S, int MODE>
 __global__ void __launch_bounds__(kReduceThreads) stencilSpmv2Kernel(StencilArgs a, const double* x, double* __restrict__ y,
                                                                       const double* w)
 {
-    chainWait();
+    chainWait(kEarlySweep);
     const unsigned nblk = cellBlocksFor(a.N);
     const unsigned lb = blockIdx.x;
     if (a.ks && a.ks->status != KS_RUNNING) return;

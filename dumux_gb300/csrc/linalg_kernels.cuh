@@ -21,6 +21,7 @@ struct SpmvArgs {
     int64_t off[7];
     KrylovState* ks;
     ReduceScratch scratch;
+    unsigned early = kEarlyWide;   // chainWait's limit; that of a batched launch is the launch's
 };
 
 template <class MT, class VT>
@@ -72,6 +73,7 @@ struct BicgArgs {
     float* rLow;
     // FP32 preconditioner output read by the x updates in place of y (x += s*yLow)
     const float* yLow;
+    unsigned early = kEarlyWide;   // chainWait's limit; that of a batched launch is the launch's
 };
 
 struct ToDoubleArgs {
@@ -218,6 +220,7 @@ void launchDefect(const DefectArgs& a, int b, int dim, cudaStream_t st);
 struct BlockMap {
     const uint2* map = nullptr;   // device array of `blocks` entries
     unsigned blocks = 0;
+    unsigned early = kEarlyWide;  // chainWait's limit of the Krylov kernels
 };
 int cellBlocks(int64_t N);
 // Host side of a block map: the entries for problems of the given lengths, blocks
