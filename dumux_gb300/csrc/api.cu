@@ -599,7 +599,11 @@ void tabulate(dxg_ctx* c, const dxg_problem_desc* d)
     c->stencilPack = StencilPackPlan{};
     c->stencilPlane = StencilPlanePlan{};
     c->packPlanned = c->packTimed = false;
-    c->packMem.release();
+    {
+        Spare::Use use(c->packSpare);
+        c->packMem.release();
+        c->packSpare.taken = false;
+    }
     c->waveTuneCount = 0;
     c->dropGraphs();   // the captured chunks hold the old buffers' addresses
     DXG_CUDA(cudaMemsetAsync(c->counters.get(), 0, 8 * sizeof(unsigned), st));
@@ -770,7 +774,11 @@ void tabulateMpfa(dxg_ctx* c, const dxg_problem_desc* d)
     c->stencilPack = StencilPackPlan{};
     c->stencilPlane = StencilPlanePlan{};
     c->packPlanned = c->packTimed = false;
-    c->packMem.release();
+    {
+        Spare::Use use(c->packSpare);
+        c->packMem.release();
+        c->packSpare.taken = false;
+    }
     c->waveTuneCount = 0;
     c->dropGraphs();
     DXG_CUDA(cudaMemsetAsync(c->counters.get(), 0, 8 * sizeof(unsigned), st));
@@ -1175,41 +1183,49 @@ void preparePack(dxg_ctx* c)
         c->packTimed = c->packPlan.ok && c->lanePlan.ok && c->packPlan.grid > kPackSureClusters * c->packPlan.clusterSize;
     }
     if (!usePack(c) || c->packMem.get()) return;
+    // what the context needs when it has to go on without the records
+    if (c->lanePlan.ok) laneHandoff<T>(c);
     const LanePackPlan& p = c->packPlan;
     const size_t records = lanePackBytes(p, 1, sizeof(T)) + lanePackBytes(p, -1, sizeof(T));
     const size_t handoff = laneHandoffBytes(p, sizeof(T));
-    try {
-        c->packMem.alloc(records + handoff);
-    } catch (const Error& e) {
-        if (e.status != DXG_ERR_OOM) throw;
-        cudaGetLastError();
-        c->packPlan.ok = false;
+    if (!c->packMem.allocSpare(records + handoff)) {
+        c->forgetPacks();
         return;
     }
+    c->packSpare.join(c->device);
     DXG_CUDA(cudaMemsetAsync(c->packMem.get() + records, 0xff, handoff, c->stream));
 }
 
-// As preparePack, for the MPFA-O stencils (2D scalar, 3D).
-void prepareStencilPack(dxg_ctx* c)
+// As preparePack, for the MPFA-O stencils (2D scalar, 3D); whether the records are to be laid.
+bool prepareStencilPack(dxg_ctx* c)
 {
+    if (c->iluKernel != DXG_ILU_AUTO) return false;   // nothing would read them
     if (!c->packPlanned) {
         c->packPlanned = true;
         c->stencilPack = makeStencilPackPlan(stencilArgs(c));
         c->stencilPlane = makeStencilPlanePlan(stencilArgs(c));
     }
-    if ((!c->stencilPack.ok && !c->stencilPlane.ok) || c->packMem.get()) return;
-    try {
-        if (c->stencilPack.ok) {
-            c->packMem.alloc(stencilPackBytes(c->stencilPack, 1) + stencilPackBytes(c->stencilPack, -1));
-        } else {
-            const StencilArgs a = stencilArgs(c);
-            c->packMem.alloc(stencilPlaneBytes(a, c->stencilPlane, 1) + stencilPlaneBytes(a, c->stencilPlane, -1));
-        }
-    } catch (const Error& e) {
-        if (e.status != DXG_ERR_OOM) throw;
-        cudaGetLastError();
-        c->stencilPack.ok = c->stencilPlane.ok = false;
+    if (!c->stencilPack.ok && !c->stencilPlane.ok) return false;
+    if (c->packMem.get()) return true;
+    const StencilArgs a = stencilArgs(c);
+    if (!c->packMem.allocSpare(c->stencilPack.ok ? stencilPackBytes(c->stencilPack, 1) + stencilPackBytes(c->stencilPack, -1)
+                                                 : stencilPlaneBytes(a, c->stencilPlane, 1) +
+                                                       stencilPlaneBytes(a, c->stencilPlane, -1))) {
+        c->forgetPacks();
+        return false;
     }
+    c->packSpare.join(c->device);
+    return true;
+}
+
+// A setting under which nothing reads the packed records gives their memory back.
+void dropUnusedPacks(dxg_ctx* c)
+{
+    if (c->mpfa ? c->iluKernel == DXG_ILU_AUTO : usePack(c)) return;
+    Spare::Use use(c->packSpare);
+    if (!c->packMem.get()) return;
+    c->packMem.release();
+    c->dropGraphs();   // the captured chunks hold its address
 }
 
 template <class T>
@@ -1391,8 +1407,7 @@ void tuneWavePlan(dxg_ctx* c, const T* A, T* L, T* Dinv, const T* in, T* out)
         DXG_CUDA(cudaEventElapsedTime(&ms, e0, e1));
         ms /= kReps;
         if ((useLane(c) && ms > c->laneTuneMs) || (c->iluKernel == DXG_ILU_AUTO && bestMs > 0.f && ms > bestMs)) {
-            c->packPlan.ok = false;
-            c->packMem.release();
+            c->forgetPacks();
         }
     }
     cudaEventDestroy(e0);
@@ -1456,6 +1471,14 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
     PT* PL = mixed ? (PT*)c->Lf.get() : (PT*)c->L.get();
     PT* PD = mixed ? (PT*)c->Dinvf.get() : (PT*)c->Dinv.get();
     IluArgs<PT, PT> ia = iluArgs<PT>(c, PA, PL, PD);
+    Spare::Use use(c->packSpare);
+    if (c->packSpare.taken) c->forgetPacks();
+    auto packStencil = [&] {
+        if (!prepareStencilPack(c)) return;
+        if (c->stencilPack.ok) launchStencilPack(stencilArgs(c), c->stencilPack, st);
+        else launchStencilPlanePack(stencilArgs(c), c->stencilPlane, st);
+        c->launches += 1;
+    };
     if (refactor) {
         TimedScope factorScope(c, DXG_KC_ILU_FACTOR, c->bytesFactor);
         if (mixed) {
@@ -1468,11 +1491,7 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
             if constexpr (!mixed) {
                 launchStencilFactor(stencilArgs(c), st);
                 c->launches += 1;
-                prepareStencilPack(c);
-                // whatever kernel is set: it may be changed without a new factor
-                if (c->stencilPack.ok) launchStencilPack(stencilArgs(c), c->stencilPack, st);
-                else if (c->stencilPlane.ok) launchStencilPlanePack(stencilArgs(c), c->stencilPlane, st);
-                c->launches += c->stencilPack.ok || c->stencilPlane.ok;
+                packStencil();
             }
         } else if (c->linearSolver == DXG_LINEAR_SOLVER_AMG_BICGSTAB) {
             // AMG setup: fine pivots, then each coarse operator (with its pivots) from the one above
@@ -1492,13 +1511,15 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
         } else {
             c->launches += launchIluFactor<PT>(ia, c->levels, c->b, c->dim, st);
         }
-        if (!c->mpfa) {
+        if (!c->mpfa && c->linearSolver == DXG_LINEAR_SOLVER_ILU_BICGSTAB) {
             preparePack<PT>(c);
             if (usePack(c)) {
                 launchLanePack<PT>(c->packPlan, packArgs<PT>(c, PA, PL, PD, nullptr, nullptr), st);
                 c->launches += 1;
             }
         }
+    } else if (c->mpfa && !c->packMem.get()) {
+        packStencil();   // the MPFA-O kernel has been changed without a new factor
     }
     double *x = c->kx.get(), *r = c->kr.get(), *rt = c->krt.get(), *p = c->kp.get(), *v = c->kv.get(),
            *t = c->kt.get(), *y = c->ky.get();
@@ -1882,6 +1903,7 @@ int dxg_ctx_create(dxg_ctx** out, int device)
 int dxg_ctx_destroy(dxg_ctx* c)
 {
     if (!c) return DXG_ERR_ARG;
+    c->packSpare.leave();
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (auto& t : c->pending) {
@@ -2174,6 +2196,7 @@ int dxg_set_ilu_kernel(dxg_ctx* c, int kind)
             return DXG_ERR_ARG;
         }
         c->iluKernel = kind;
+        dropUnusedPacks(c);
         return DXG_OK;
     }
     if (kind == DXG_ILU_WAVEFRONT && c->uploaded && !c->wavePlan.ok) {
@@ -2186,6 +2209,7 @@ int dxg_set_ilu_kernel(dxg_ctx* c, int kind)
     }
     c->iluKernel = kind;
     c->haveFactor = false;
+    dropUnusedPacks(c);
     return DXG_OK;
 }
 
@@ -2201,6 +2225,7 @@ int dxg_set_lane_ring(dxg_ctx* c, int form)
     c->waveTuned = false;
     c->haveFactor = false;
     c->dropGraphs();
+    dropUnusedPacks(c);
     return DXG_OK;
 }
 
@@ -2221,6 +2246,7 @@ int dxg_set_linear_solver(dxg_ctx* c, int kind)
     }
     c->linearSolver = kind;
     c->haveFactor = false;
+    dropUnusedPacks(c);
     return DXG_OK;
 }
 

@@ -115,7 +115,7 @@ struct Arena {
             Block b;
             b.cap = std::max<size_t>(need, 4u << 20);
             DXG_CUDA(cudaMallocHost(&b.host, b.cap));
-            if (cudaMalloc(&b.dev, b.cap) != cudaSuccess) {
+            if (deviceMalloc(reinterpret_cast<void**>(&b.dev), b.cap) != cudaSuccess) {
                 cudaGetLastError();
                 cudaFreeHost(b.host);
                 throw Error(DXG_ERR_OOM, "argument arena allocation failed");
@@ -191,7 +191,14 @@ struct dxg_batch {
     bool amg = false;                 // AMG-BiCGSTAB instead of ILU(0)-BiCGSTAB
     int64_t budget = 0, bytesInUse = 0;
     int64_t packBytes = 0;            // packed factor records of the members (extra to bytesInUse)
-    bool noPacks = false;             // the device memory did not hold them
+    bool noPacks = false;             // the device memory did not hold them, or was needed elsewhere
+    struct PackSpare : Spare {
+        dxg_batch* b;
+        explicit PackSpare(dxg_batch* batch) : b(batch) {}
+        ~PackSpare() override { leave(); }
+        bool give() override;
+    };
+    mutable PackSpare packSpare{this};
     int64_t nextId = 1;
     int64_t launches = 0;
     std::map<int64_t, std::unique_ptr<Slot>> slots;
@@ -868,6 +875,22 @@ void dropPacks(dxg_batch* B)
     B->packBytes = 0;
 }
 
+}  // namespace
+
+// The packed records are needed elsewhere (the batch is between two calls).
+bool dxg_batch::PackSpare::give()
+{
+    if (b->packBytes == 0) return false;
+    try {
+        dropPacks(b);
+    } catch (const Error&) {
+        return false;
+    }
+    return b->noPacks = true;
+}
+
+namespace {
+
 // Which members share a launch: first fit over the members by falling length of their sweeps.
 template <class PT>
 std::vector<std::vector<uint2>> packRounds(const Members& S, int warps, size_t smem)
@@ -931,15 +954,12 @@ bool preparePacks(dxg_batch* B, const Members& S)
         dxg_ctx* c = s->c;
         if (c->packMem.get()) continue;
         const size_t bytes = bytesOf(c->packPlan), handoff = laneHandoffBytes(c->packPlan, sizeof(PT));
-        try {
-            c->packMem.alloc(bytes);
-        } catch (const Error& e) {
-            if (e.status != DXG_ERR_OOM) throw;
-            cudaGetLastError();
+        if (!c->packMem.allocSpare(bytes)) {
             dropPacks(B);
             B->noPacks = true;
             return false;
         }
+        B->packSpare.join(B->device);
         B->packBytes += (int64_t)bytes;
         DXG_CUDA(cudaMemsetAsync(c->packMem.get() + bytes - handoff, 0xff, handoff, B->stream));
     }
@@ -1714,6 +1734,7 @@ int dxg_batch_create(dxg_batch** out, int device, int precision)
 int dxg_batch_destroy(dxg_batch* b)
 {
     if (!b) return DXG_ERR_ARG;
+    b->packSpare.leave();
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (auto& t : b->pending) {
@@ -1785,6 +1806,7 @@ int64_t dxg_problem_device_bytes(const dxg_problem_desc* d, int precision)
 int dxg_batch_set_memory_budget(dxg_batch* b, int64_t bytes)
 {
     if (!b || bytes < 0) return DXG_ERR_ARG;
+    Spare::Use use(b->packSpare);
     b->budget = bytes;
     // the packed records give way to the problems
     if (bytes > 0 && b->bytesInUse + b->packBytes > bytes)
@@ -1802,6 +1824,7 @@ int dxg_batch_add(dxg_batch* b, const dxg_problem_desc* d, const double* u0, dou
                   double t_end, const dxg_newton_params* params, int64_t* id)
 {
     if (!b || !d || !u0 || !id) return DXG_ERR_ARG;
+    Spare::Use use(b->packSpare);
     if (d->discretization != DXG_DISC_TPFA) {
         b->err = "batched problems use the TPFA discretization";
         return DXG_ERR_ARG;
@@ -1874,6 +1897,7 @@ int dxg_batch_add(dxg_batch* b, const dxg_problem_desc* d, const double* u0, dou
 int dxg_batch_iterate(dxg_batch* b, int32_t* active)
 {
     if (!b) return DXG_ERR_ARG;
+    Spare::Use use(b->packSpare);
     return guardedB(b, [&] {
         DXG_CUDA(cudaSetDevice(b->device));
         std::map<GroupKey, Members> groups;
@@ -1945,6 +1969,7 @@ int dxg_batch_remove(dxg_batch* b, int64_t id)
     if (!b) return DXG_ERR_ARG;
     auto it = b->slots.find(id);
     if (it == b->slots.end()) return DXG_ERR_ARG;
+    Spare::Use use(b->packSpare);
     cudaSetDevice(b->device);
     cudaStreamSynchronize(b->stream);
     b->bytesInUse -= it->second->bytes;
@@ -1958,6 +1983,7 @@ int64_t dxg_batch_launch_count(const dxg_batch* b) { return b ? b->launches : -1
 int dxg_batch_describe(const dxg_batch* b, char* buf, int64_t len)
 {
     if (!b || !buf || len <= 0) return DXG_ERR_ARG;
+    Spare::Use use(b->packSpare);
     std::string out;
     for (const auto& kv : b->groups) {
         const GroupKey& k = kv.first;

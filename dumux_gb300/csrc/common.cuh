@@ -9,6 +9,7 @@
 #include <utility>
 
 #include "../../include/dumux_gb300.h"
+#include "spare.h"
 
 namespace dxg {
 
@@ -76,8 +77,21 @@ struct DevBuf {
             n = count;
             return;
         }
-        DXG_CUDA(cudaMalloc(&p, count * sizeof(T)));
+        DXG_CUDA(deviceMalloc(reinterpret_cast<void**>(&p), count * sizeof(T)));
         n = count;
+    }
+    // memory that the owner can do without (spare.h): false where the device does not have it to spare
+    bool allocSpare(size_t count)
+    {
+        release();
+        const cudaError_t e = spareMalloc(reinterpret_cast<void**>(&p), count * sizeof(T));
+        if (e == cudaErrorMemoryAllocation) {
+            p = nullptr;
+            return false;
+        }
+        DXG_CUDA(e);
+        n = count;
+        return true;
     }
     T* get() const { return p; }
     size_t bytes() const { return n * sizeof(T); }

@@ -126,6 +126,27 @@ struct dxg_ctx {
     bool packPlanned = false;
     bool packTimed = false;               // the TPFA plan is timed against the others at the first factorisation
     dxg::DevBuf<unsigned char> packMem;   // records of both sweeps, then the hand-off buffer
+    // ... which the context gives back when device memory runs out elsewhere, and then does without
+    struct PackSpare : dxg::Spare {
+        dxg_ctx* c;
+        bool taken = false;
+        explicit PackSpare(dxg_ctx* ctx) : c(ctx) {}
+        ~PackSpare() override { leave(); }
+        bool give() override
+        {
+            if (!c->packMem.get()) return false;
+            c->packMem.release();
+            return taken = true;
+        }
+    };
+    PackSpare packSpare{this};
+    void forgetPacks()
+    {
+        packPlan.ok = stencilPack.ok = stencilPlane.ok = false;
+        packMem.release();
+        packSpare.taken = false;
+        dropGraphs();
+    }
     dxg::DevBuf<unsigned char> laneHandoff;
     size_t laneHandoffBytes = 0;
     // limit of every bounded wait of the sweeps (0: the kernels' default, 0.5 s)

@@ -267,8 +267,10 @@ enum { DXG_ILU_AUTO = 0, DXG_ILU_WAVEFRONT = 1, DXG_ILU_LEVELS = 2, DXG_ILU_REDB
 /* DXG_ILU_LANES: the natural-order sweeps with one lane per grid line and block row, tiles of a
  * z-plane per CTA over several thread-block clusters (more SMs on the level chain); the same
  * factors and arithmetic per cell as DXG_ILU_WAVEFRONT, so the same results.  The factor is
- * re-laid for them after each factorisation, which takes about its size in device memory more;
- * where that is not there, the sweeps read the factor in place. */
+ * re-laid for them after each factorisation, which takes about its size in device memory more.
+ * That memory is spare: it is taken only where 64 MB stay free beside it, given back under a setting
+ * that does not read it, and given back for good (until the next upload) when another context or
+ * batch of the process finds the device full.  Without it the sweeps read the factor in place. */
 int dxg_set_ilu_kernel(dxg_ctx* ctx, int kind);
 /* Form of the lane sweeps: 0 (default) the packed records where they fit, else the faster of the
  * two forms that read the factor in place, timed at the first factorisation; 1 the register form
@@ -405,12 +407,14 @@ const char* dxg_batch_last_error(const dxg_batch* batch);
  * context) for every problem of the batch, each V-cycle pass batched over the problems
  * that have that level (default 0); set before the first dxg_batch_add. */
 int dxg_batch_set_option(dxg_batch* batch, int option, int value);
-/* Device memory that admitting this problem takes (tables and all solver state). */
+/* Device memory that admitting this problem takes (tables and all solver state).  The packed factor
+ * records of DXG_ILU_AUTO and DXG_ILU_LANES are no part of it: they are spare memory, which gives way. */
 int64_t dxg_problem_device_bytes(const dxg_problem_desc* desc, int precision);
 /* Admission limit on the device memory of all admitted problems (0: unlimited).
  * dxg_batch_add refuses with DXG_ERR_BUDGET a problem that would exceed it.  The packed factor
  * records of the natural-order sweeps (about another factor per problem) are no part of a
- * problem's bytes; they are made within what a limit leaves and given back for admissions. */
+ * problem's bytes; they are made within what a limit leaves and given back for admissions, and when
+ * another context or batch of the process finds the device full. */
 int dxg_batch_set_memory_budget(dxg_batch* batch, int64_t bytes);
 int64_t dxg_batch_device_bytes(const dxg_batch* batch);
 /* Admit a problem: initial solution u0 (N*num_eq values, also the first previous
