@@ -358,3 +358,41 @@ def test_wait_limit_is_that_of_a_single_wait(kind, limit):
     ctx.set_wait_limit(limit)
     assert ctx.linear_solve(1e-6, 60) == first
     assert np.array_equal(ctx.update(), x0)
+
+
+# the one-CTA line sweeps, which 2D grids run where their packed plan does not fit (long lines) or the
+# records are not to be had: one to sixteen warps of lines
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("eqs,dims", [(1, (1, 1)), (1, (13, 11)), (1, (9, 512)), (1, (1000, 8)), (2, (13, 11)),
+                                      (2, (100, 100)), (2, (37, 300)), (2, (700, 20))])
+def test_line_sweeps_equal_cluster_wavefront(eqs, dims, precision):
+    if eqs == 1:
+        desc, u = problems.darcy_1p(cells=dims, seed=4)
+        prev, dt = u, 0.0
+    else:
+        desc, prev = problems.dnapl_2p(cells=dims, extent=(6.0, 4.0), seed=4)
+        u = prev.reshape(-1, 2).copy()
+        u[:, 1] = np.random.default_rng(3).uniform(0.0, 0.3, len(u))
+        u, dt = u.reshape(-1), 250.0
+    n0, x0, _ = _solve(desc, u, prev, "wavefront", precision, dt)
+    ctx = Context(desc, precision=precision)
+    ctx.set_ilu_kernel("lanes")
+    ctx.set_lane_ring("registers")
+    ctx.set_solution(u)
+    if dt:
+        ctx.set_prev_solution(prev)
+        ctx.set_time_step(dt)
+    ctx.assemble_jacobian_and_residual()
+    n1 = ctx.linear_solve(1e-10 if precision == "fp64" else 1e-4, 400)["iterations"]
+    assert "line sweeps in one CTA" in ctx.describe()
+    assert n1 == n0
+    assert np.array_equal(ctx.update(), x0)
+
+
+def test_long_lines_do_not_fit_the_packed_plan():
+    desc, u = problems.darcy_1p(cells=(1000, 8), seed=4)
+    n0, x0, _ = _solve(desc, u, u, "wavefront", "fp64", 0.0)
+    for kind in ("auto", "lanes"):
+        n1, x1, how = _solve(desc, u, u, kind, "fp64", 0.0)
+        assert "packed records" not in how
+        assert n1 == n0 and np.array_equal(x1, x0)
