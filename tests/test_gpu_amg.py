@@ -11,7 +11,7 @@ import pytest
 import scipy.sparse as sp
 
 import oracle
-from dumux_gb300 import Context, newton_params, problems
+from dumux_gb300 import Batch, Context, newton_params, problems
 
 pytestmark = pytest.mark.gpu
 
@@ -243,3 +243,33 @@ def test_amg_continuous_batching_mixed_kinds_equal_alone():
                 ctx.advance_time_step()
                 cur = min(ctx.suggest_time_step(rep["dt_used"], params), dt, t_end - t)
         assert np.array_equal(batch.solution(pid), ctx.solution()), (desc.cells, desc.num_eq)
+
+
+# the branches of the small levels' cluster cycle: one level alone (the direct solve), one level above
+# it, top levels of fewer cells than the CTAs hold, second levels too large for one CTA (the cycle
+# starts further down) and long thin grids; a batch runs every level's passes from global memory
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("eqs", [1, 2])
+@pytest.mark.parametrize("dims", [(1, 1), (8, 8), (4, 4, 4), (5, 1, 3), (65, 1), (13, 5), (9, 9), (17, 16, 16),
+                                  (4096, 1), (1000, 2, 2), (2, 3, 600), (40, 30, 20)])
+def test_amg_small_levels_equal_batched_passes(dims, eqs, precision):
+    p = newton_params(linear_max_iter=500)
+    if eqs == 1:
+        desc, u0 = problems.darcy_1p(cells=dims, seed=3)
+    else:
+        desc, u0 = problems.dnapl_2p(cells=dims, extent=(6.0, 4.0, 1.0)[:len(dims)], seed=3)
+    dt = 250.0 if eqs == 2 else 0.0
+    batch = Batch(precision=precision, solver="amg")
+    i = batch.add(desc, u0, dt=dt, t_end=dt, params=p)
+    batch.run()
+    ctx = Context(desc, precision=precision)
+    ctx.set_linear_solver("amg")
+    ctx.set_solution(u0)
+    ctx.set_prev_solution(u0)
+    # (1000x2x2 2p: no step length down to dt / 1024 brings Newton to converge, in either)
+    rep = ctx.newton_solve(dt, p, raise_on_failure=False)
+    assert batch.info(i)["status"] == rep["status"]
+    if rep["status"] == 0:
+        assert rep["time_step_divisions"] == batch.info(i)["time_step_divisions"]
+        assert batch.info(i)["linear_iterations"] == rep["linear_iterations"]
+        assert np.array_equal(batch.solution(i), ctx.solution())
