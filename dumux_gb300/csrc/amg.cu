@@ -329,12 +329,20 @@ __global__ void amgRestrictKernel(AmgLevel<T> F, AmgLevel<T> C, const KrylovStat
 constexpr int kAmgMaxClusterLevels = 12;
 constexpr int kAmgClusterCtas = 16;
 constexpr int kAmgClusterThreads = 512;
-// Largest second level, in cells.  A time step with the cluster launch from the level above it, and
-// from that level itself, against all small levels in one cluster launch out of global memory: FP64
-// 40x30x20 (second level of 400 cells) 42.5 and 38.6 ms against 43.9; FP32 41x30x20 (440) 23.9 and
-// 25.4 against 26.8, 70x58x8 (540) 15.9 and 16.3 against 16.4.
+// Largest second level, in cells, for the cycle to start from the level above it.  A BiCGSTAB iteration
+// in us, started there and started from the second level itself, 2x2 blocks: FP64 245 cells (grid
+// 14x14x10) 131 and 136, 256 (16x16x8) 123 and 129, 256 (64x64x32) 259 and 259, 288 (18x16x8) 134 and
+// 130, 512 (16x16x16) 193 and 138; FP32 500 (40x40x20) 129 and 133, 512 98 and 104, 625 (50x50) 93 and
+// 120, 1024 (64x64) 104 and 119.  Beyond the lines 1x1 blocks and FP32 could still take it: FP64 1x1 512
+// cells 88 and 91, 1024 103 and 109.
 constexpr int64_t kAmgOneCtaLevel64 = 256, kAmgOneCtaLevel32 = 640;
 constexpr size_t kAmgClusterSmem = 220 * 1024;
+// What the cycle holds without the matrices of the lower levels always fits: a sixteenth of the top
+// level with its matrix (3D, 2x2 blocks: 40 elements a cell), and the levels below, 12 elements a cell
+// of a second level that is limited, each further one about half of the one before at most.
+static_assert((kAmgClusterLevel / kAmgClusterCtas * 40 + 3 * kAmgOneCtaLevel64 * 12) * 8 <= (int64_t)kAmgClusterSmem &&
+                  (kAmgClusterLevel / kAmgClusterCtas * 40 + 3 * kAmgOneCtaLevel32 * 12) * 4 <= (int64_t)kAmgClusterSmem,
+              "");
 template <class T>
 struct AmgCycle {
     AmgLevel<T> lv[kAmgMaxClusterLevels];
@@ -782,18 +790,14 @@ int64_t vcycle(const std::vector<AmgLevel<T>>& Ls, size_t l, const KrylovState* 
 {
     const AmgLevel<T>& L = Ls[l];
     const unsigned g = gridFor(L.N);
-    size_t elems = 0;
     // the level after the top one runs in one CTA: where it is large, in FP64 above all, a pass costs
     // that SM more than a launch spread over the GPU, and the cluster starts a level further down
     const bool oneCta = l + 1 >= Ls.size() || Ls[l + 1].N <= (sizeof(T) == 8 ? kAmgOneCtaLevel64 : kAmgOneCtaLevel32);
     if (L.N <= kAmgClusterLevel && Ls.size() - l <= (size_t)kAmgMaxClusterLevels && oneCta) {
-        const size_t last = Ls.size() - 1;
-        elems = last > l ? amgTopElems<B, DIM, T>(L.N) : 0;
-        for (size_t k = last > l ? l + 1 : l; k <= last; ++k) elems += amgSubElems<B, DIM, T>(Ls[k].N, k == last, false);
-        if (elems * sizeof(T) > kAmgClusterSmem) elems = 0;   // long thin grids: from a level further down
-    }
-    if (elems > 0) {
         // this level and all below: one cluster launch
+        const size_t last = Ls.size() - 1;
+        size_t elems = last > l ? amgTopElems<B, DIM, T>(L.N) : 0;
+        for (size_t k = last > l ? l + 1 : l; k <= last; ++k) elems += amgSubElems<B, DIM, T>(Ls[k].N, k == last, false);
         AmgCycle<T> cy{};
         cy.count = (int)(Ls.size() - l);
         for (int k = 0; k < cy.count; ++k) cy.lv[k] = Ls[l + k];
