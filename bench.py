@@ -70,8 +70,9 @@ def parse():
                     help="Jacobian by numeric differentiation (default, the reference's default) or analytic")
     ap.add_argument("--ilu", default="natural", choices=["natural", "lanes", "wavefront", "redblack"],
                     help="ILU(0) of the single-problem workloads: natural order (the reference's SeqILU, "
-                         "default; lane sweeps over packed records where they fit), natural order forced onto the lane sweeps or onto the cluster "
-                         "wavefront, or red-black (two parallel passes per sweep, more iterations)")
+                         "default; lane sweeps over packed records where they fit), natural order forced onto "
+                         "the lane sweeps or onto the cluster wavefront, or red-black (two parallel passes "
+                         "per sweep, more iterations)")
     ap.add_argument("--solver", default="ilu", choices=["ilu", "amg"],
                     help="ILU(0)-BiCGSTAB (default, the reference's ILUBiCGSTABIstlSolver) or "
                          "AMG-BiCGSTAB (AMGBiCGSTABIstlSolver)")

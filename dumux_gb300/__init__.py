@@ -262,8 +262,9 @@ class Context:
     def set_ilu_kernel(self, kind):
         """'auto' (lane sweeps over packed records where they fit, else the fastest), 'wavefront'
         (one cluster launch per sweep), 'lanes' (one lane per grid line and block row, tiles of a
-        plane per CTA over several clusters) or 'levels' (one launch per level): the natural-order ILU(0) of the reference; 'redblack': ILU(0) of the red-black
-        reordered matrix (a different preconditioner, two parallel passes per sweep)."""
+        plane per CTA over several clusters) or 'levels' (one launch per level): the natural-order
+        ILU(0) of the reference; 'redblack': ILU(0) of the red-black reordered matrix (a different
+        preconditioner, two parallel passes per sweep)."""
         self._check(self._L.dxg_set_ilu_kernel(self._h, {"auto": 0, "wavefront": 1, "levels": 2,
                                                           "redblack": 3, "lanes": 4}[kind]))
 

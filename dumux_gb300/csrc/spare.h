@@ -111,15 +111,18 @@ inline cudaError_t deviceMalloc(void** p, size_t bytes)
 }
 
 // Spare memory is taken only while this much stays free beside it, for what the driver and the
-// library allocate in small pieces (graphs, kernels loaded on first use, argument blocks).
-constexpr size_t kSpareHeadroom = 64u << 20;
+// library allocate in small pieces (graphs, kernels loaded on first use, argument blocks); small
+// pieces of its own without asking, which would take a small problem's first solve 40 us.
+constexpr size_t kSpareHeadroom = 64u << 20, kSpareSmall = 1u << 20;
 inline cudaError_t spareMalloc(void** p, size_t bytes)
 {
-    size_t free = 0, total = 0;
-    cudaError_t e = cudaMemGetInfo(&free, &total);
-    if (e != cudaSuccess) return e;
-    if (free < bytes + kSpareHeadroom) return cudaErrorMemoryAllocation;
-    e = cudaMalloc(p, bytes);
+    if (bytes > kSpareSmall) {
+        size_t free = 0, total = 0;
+        const cudaError_t e = cudaMemGetInfo(&free, &total);
+        if (e != cudaSuccess) return e;
+        if (free < bytes + kSpareHeadroom) return cudaErrorMemoryAllocation;
+    }
+    const cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) cudaGetLastError();
     return e;
 }

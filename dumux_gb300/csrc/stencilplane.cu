@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kPlRoles * kPlMaxTiles * 32) stencilPlaneApply
             }
         };
         sweep(std::integral_constant<int, 1>{});
-        // the first warps read the second warps' forward results
+        // role 0 reads the forward results of role 3
         asm volatile("bar.sync 1, %0;" ::"r"(kPlRoles * W * 32) : "memory");
         sweep(std::integral_constant<int, -1>{});
     }

@@ -280,10 +280,10 @@ int dxg_set_ilu_kernel(dxg_ctx* ctx, int kind);
  * counterpart in the reference. */
 int dxg_set_lane_ring(dxg_ctx* ctx, int form);
 /* Limit of every bounded wait inside the ILU(0) sweeps, in seconds (default 0.5; at most
- * 60).  A wait that runs out ends the sweep with DXG_ERR_TIMEOUT, which the Newton driver
- * treats like a failed linear solve (a time-step retry).  Raise it where the GPU is
- * time-sliced with other processes, whose turns can stall a sweep for longer.  No
- * counterpart in the reference (its sweeps run on one CPU thread). */
+ * 60); it counts for each wait by itself.  A wait that runs out ends the sweep, and the linear or
+ * Newton solve with it, with DXG_ERR_TIMEOUT.  Raise it where the GPU is time-sliced with other
+ * processes, whose turns can stall a sweep for longer.  No counterpart in the reference (its sweeps
+ * run on one CPU thread). */
 int dxg_set_wait_limit(dxg_ctx* ctx, double seconds);
 /* The linear solver of dxg_linear_solve / dxg_newton_solve, as the reference's solver
  * types: DXG_LINEAR_SOLVER_ILU_BICGSTAB (ILUBiCGSTABIstlSolver, istlsolvers.hh:635-642;
