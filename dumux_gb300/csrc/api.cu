@@ -1671,6 +1671,7 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
         }
         DXG_CUDA(cudaMemsetAsync(c->singular.get() + 1, 0, sizeof(int), st));
         DXG_CUDA(cudaStreamSynchronize(st));
+        if (flags[1] == DXG_ERR_CUDA) throw Error(DXG_ERR_CUDA, "lane sweeps were run without their thread-block clusters");
         throw Error(DXG_ERR_TIMEOUT, "ILU(0) wavefront wait timed out");
     }
     const KrylovState& ks = *c->ksHost;

@@ -222,6 +222,13 @@ __global__ void __launch_bounds__((kLpMaxWarps + 1) * 32) lanePackApply(LanePack
     __shared__ __align__(8) unsigned long long bars[kLpMaxWarps][kLpMaxStages];
 
     cg::cluster_group cluster = cg::this_cluster();
+    // Every hand-off inside a cluster goes to a rank of the plan's: launched with other clusters (by a
+    // tool that repeats the launch without its attributes) the kernel does nothing and says so.
+    if (cluster.num_blocks() != (unsigned)a.clusterSize) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (threadIdx.x == 0) atomicExch(a.err, DXG_ERR_CUDA);
+        return;
+    }
     const int nx = a.nx, ny = a.ny, W = a.warps, steps = a.steps, stages = a.stages;
     const LpSmem lay = lpSmem(steps, W, stages, SS, B, R, DIM, TS);
     const int cta = (int)who.y;
