@@ -1458,6 +1458,9 @@ IluArgs<T, T> iluArgs(dxg_ctx* c, const T* A, T* L, T* Dinv)
     return a;
 }
 
+// The packed sweeps found themselves launched without their thread-block clusters.
+struct ClustersLost {};
+
 // BiCGSTAB with ILU(0) on the device from x = 0 for rhs (FP64 in device memory):
 // Krylov vectors and SpMV in FP64 on the FP64 Jacobian; the ILU(0) preconditioner in
 // PT -- FP64 (plain path) or FP32 (mixed precision: FP32 copy of the Jacobian, FP32
@@ -1671,7 +1674,7 @@ dxg_linear_result bicgstab(dxg_ctx* c, const double* rhs, double reduction, int 
         }
         DXG_CUDA(cudaMemsetAsync(c->singular.get() + 1, 0, sizeof(int), st));
         DXG_CUDA(cudaStreamSynchronize(st));
-        if (flags[1] == DXG_ERR_CUDA) throw Error(DXG_ERR_CUDA, "lane sweeps were run without their thread-block clusters");
+        if (flags[1] == DXG_ERR_CUDA) throw ClustersLost{};
         throw Error(DXG_ERR_TIMEOUT, "ILU(0) wavefront wait timed out");
     }
     const KrylovState& ks = *c->ksHost;
@@ -1695,9 +1698,21 @@ dxg_linear_result linearSolve(dxg_ctx* c, double reduction, int maxit)
 {
     requireUploaded(c);
     if (!c->haveJac || !c->haveRes) throw Error(DXG_ERR_STATE, "assemble before solving");
-    dxg_linear_result res = c->precision == DXG_PRECISION_FP64
-                                ? bicgstab<double>(c, c->r.get(), reduction, maxit, !c->haveFactor)
-                                : bicgstab<float>(c, c->r.get(), reduction, maxit, !c->haveFactor);
+    auto solve = [&] {
+        return c->precision == DXG_PRECISION_FP64 ? bicgstab<double>(c, c->r.get(), reduction, maxit, !c->haveFactor)
+                                                  : bicgstab<float>(c, c->r.get(), reduction, maxit, !c->haveFactor);
+    };
+    dxg_linear_result res;
+    try {
+        res = solve();
+    } catch (const ClustersLost&) {
+        // under a tool that repeats the launches without their clusters: without the packed sweeps
+        {
+            Spare::Use use(c->packSpare);
+            c->forgetPacks();
+        }
+        res = solve();
+    }
     c->haveFactor = true;
     DXG_CUDA(cudaMemcpyAsync(c->delta.get(), c->kx.get(), c->M * sizeof(double), cudaMemcpyDeviceToDevice,
                              c->stream));

@@ -1522,6 +1522,15 @@ void tickGroup(dxg_batch* B, const GroupKey& key, const Members& S)
     runChunk<PT>(B, G, n, dim, b);
     gather(B, S);
 
+    // packed sweeps launched without their clusters (by a tool that repeats the launches): every member
+    // begins its iteration anew, without them
+    for (int k = 0; k < n; ++k)
+        if (B->reportsHost[k].timeout == DXG_ERR_CUDA) {
+            for (Slot* s : S) s->solving = false;
+            B->noPacks = true;
+            dropPacks(B);
+            return;
+        }
     Members U;
     std::vector<int> ended;
     for (int k = 0; k < n; ++k) {

@@ -222,8 +222,9 @@ __global__ void __launch_bounds__((kLpMaxWarps + 1) * 32) lanePackApply(LanePack
     __shared__ __align__(8) unsigned long long bars[kLpMaxWarps][kLpMaxStages];
 
     cg::cluster_group cluster = cg::this_cluster();
-    // Every hand-off inside a cluster goes to a rank of the plan's: launched with other clusters (by a
-    // tool that repeats the launch without its attributes) the kernel does nothing and says so.
+    // Every hand-off inside a cluster goes to a rank of the plan's: launched with other clusters (a
+    // profiler repeats a cooperative launch without its cluster dimension) the kernel does nothing and
+    // says so, and the solve goes on with the sweeps that read the factor in place.
     if (cluster.num_blocks() != (unsigned)a.clusterSize) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (threadIdx.x == 0) atomicExch(a.err, DXG_ERR_CUDA);
